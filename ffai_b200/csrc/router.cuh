@@ -116,9 +116,53 @@ FFAI_DEVINL void warp_argbest(float& v, int& i) {
 }
 
 // Top-k of vals[0..E) in shared memory by one warp; selected indices (in
-// selection order) returned lane-wise: lane j < k holds index j.  `taken` is a
-// per-lane bit mask over the lane's strided elements (e = lane + 32*j).
+// selection order) returned lane-wise: lane j < k holds index j.
+//
+// Up to 32 * NV values: every lane keeps its strided values (e = lane + 32 j) as order-preserving integer keys in
+// registers and a round is two warp reductions in hardware (largest key, then smallest index among its holders);
+// re-reading shared memory and shuffling value and index through five steps took about five times as long.
+template <int NV>
+FFAI_DEVINL void warp_topk_regs(const float* vals, int E, int k, int lane, int& my_idx, float& my_val) {
+    uint32_t key[NV];
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const int e = lane + 32 * j;
+        key[j] = 0u;
+        if (e < E) {
+            const uint32_t b = __float_as_uint(vals[e] + 0.0f);   // -0 and +0 are one value
+            key[j] = max((b & 0x80000000u) ? ~b : (b | 0x80000000u), 1u);
+        }
+    }
+    uint32_t best = 0u, at = 0x7FFFFFFFu;
+    auto local_best = [&]() {
+        best = 0u; at = 0x7FFFFFFFu;
+#pragma unroll
+        for (int j = 0; j < NV; ++j)
+            if (key[j] > best) { best = key[j]; at = (uint32_t)(lane + 32 * j); }
+    };
+    local_best();
+    my_idx = 0;
+    my_val = 0.0f;
+    for (int r = 0; r < k; ++r) {
+        const uint32_t top = __reduce_max_sync(0xFFFFFFFFu, best);
+        const uint32_t i = __reduce_min_sync(0xFFFFFFFFu, best == top ? at : 0x7FFFFFFFu);
+        if (lane == r) my_idx = (int)i;
+        if (at == i) {
+#pragma unroll
+            for (int j = 0; j < NV; ++j)
+                if ((uint32_t)(lane + 32 * j) == i) key[j] = 0u;
+            local_best();
+        }
+    }
+    my_idx = min(my_idx, E - 1);
+    if (lane < k) my_val = vals[my_idx];
+}
+
+// The general form; `taken` is a per-lane bit mask over the lane's strided elements.
 FFAI_DEVINL void warp_topk(const float* vals, int E, int k, int lane, int& my_idx, float& my_val) {
+    if (E <= 32) { warp_topk_regs<1>(vals, E, k, lane, my_idx, my_val); return; }
+    if (E <= 128) { warp_topk_regs<4>(vals, E, k, lane, my_idx, my_val); return; }
+    if (E <= 256) { warp_topk_regs<8>(vals, E, k, lane, my_idx, my_val); return; }
     uint32_t taken = 0;
     my_idx = -1;
     my_val = 0.0f;

@@ -302,7 +302,9 @@ FFAI_API uint32_t ffai_ep_plan_exchange(const uint32_t* recv_counts, int32_t wor
  *                  overlap the compute (same bits: tokens are independent), 1 = always as one piece, 2..4 = at
  *                  most that many chunks
  *   "ksplit"       cp.async decode kernels: slices of the reduction axis per 16-row block (0 automatic, 1, 2, 4)
- *   "decode"       decode kernels: 0 automatic, 1 cp.async rings, 2 bulk-copy streams
+ *   "decode"       decode kernels: 0 automatic (up to 8 tokens and 64 routed rows, 4- and 8-bit experts: the whole block in
+ *                  one launch, unless stage timing is on or "ksplit" / "decode_team" is set), 1 cp.async rings, 2 bulk-copy
+ *                  streams
  *   "decode_team"  bulk-copy streams: warps that share one 16-row block (0 automatic, 1, 4, 16)
  *   "nt2_cost"     bulk-copy streams: schedule weight of a block with more than 8 rows, 8 = as one with fewer (8..32)
  *   "overlap"      shared expert on a second stream beside router, plan and row exchange (default 1; 0: one stream)

@@ -491,3 +491,42 @@ def test_nemotronh_style_block(oracle_mod, T):
 def test_nemotronh_style_block_other_widths(oracle_mod):
     run_and_check(oracle_mod, synth.nemotronh_style().with_(name="nemotronh_8bit", expert_bits=8, shared_bits=8, norm_topk_prob=0), 33)
     run_and_check(oracle_mod, synth.nemotronh_style().with_(name="nemotronh_no_shared", shared_intermediate=0, top_k=1), 20)
+
+
+# ── the one-launch forward of the smallest batches ──
+
+FUSED = [
+    # name, T, spec changes.  H = 64 / I = 64 (one cell, ranges with fewer cells than warps), H = 1280 (whole rounds of down
+    # items), H = 4672 (292 items: two rounds or a split axis), 64 routed rows (most) and 72 (one more token-slot row than
+    # fits: the launch chain), every code width and group the kernel takes, one expert, shared experts of both widths
+    ("smallest", 1, dict(hidden=64, intermediate=64, n_experts=1, top_k=1)),
+    ("one_cell", 8, dict(hidden=64, intermediate=64, n_experts=8, top_k=8)),
+    ("full_rows", 8, dict(hidden=512, intermediate=192, n_experts=40, top_k=8)),
+    ("too_many_rows", 8, dict(hidden=512, intermediate=192, n_experts=40, top_k=9)),
+    ("nine_tokens", 9, dict(hidden=512, intermediate=192, n_experts=40, top_k=4)),
+    ("split_down", 7, dict(hidden=4672, intermediate=704, n_experts=12, top_k=5, expert_row_bias=1)),
+    ("wide_router", 3, dict(hidden=256, intermediate=128, n_experts=300, top_k=20)),
+    ("g128", 5, dict(hidden=1280, intermediate=384, n_experts=16, top_k=4, expert_group_size=128, expert_row_bias=1)),
+    ("g32", 6, dict(hidden=1280, intermediate=320, n_experts=16, top_k=4, expert_group_size=32, expert_row_bias=1)),
+    ("b8_g32", 2, dict(hidden=512, intermediate=320, n_experts=16, top_k=4, expert_bits=8, expert_group_size=32)),
+    ("b8_g64_shared4", 4, dict(hidden=512, intermediate=320, n_experts=16, top_k=4, expert_bits=8, shared_intermediate=128, shared_bits=4,
+                               shared_group_size=64, shared_gate_kind=capi.LINEAR_BF16)),
+    ("b4_g32_shared8", 8, dict(hidden=512, intermediate=320, n_experts=16, top_k=2, expert_group_size=32, shared_intermediate=384, shared_bits=8,
+                               shared_group_size=128, shared_gate_kind=capi.LINEAR_F32)),
+    ("shared_ungated", 1, dict(hidden=2048, intermediate=64, n_experts=16, top_k=1, shared_intermediate=64, shared_bits=8, shared_group_size=64)),
+]
+
+
+@pytest.mark.parametrize("residual", [False, True])
+@pytest.mark.parametrize("name,T,kw", FUSED, ids=[f[0] for f in FUSED])
+def test_one_launch_decode(oracle_mod, name, T, kw, residual):
+    spec = synth.LayerSpec(name, **kw)
+    host = synth.make_layer(spec, 11)
+    layer = MoELayer(host, 12)
+    try:
+        for seed in (1, 2):     # the barrier word and the tickets come back to their start
+            run_and_check(oracle_mod, spec, T, seed=seed, residual=residual, layer=layer, host=host)
+        fused = T <= 8 and T * spec.top_k <= 64
+        assert (layer.launch_count() == 1) == fused
+    finally:
+        layer.close()
