@@ -1074,7 +1074,10 @@ extern "C" FFAI_API int ffai_moe_set_weights(ffai_moe_layer* L, const ffai_moe_w
             const size_t count = n * (N / 16) * (K / 64);
             if (count >= (1u << 31)) return FFAI_OK;   // the layer then keeps to the launch chain
             void* buf = nullptr;
-            CUDA_TRY(L, cudaMalloc(&buf, count * (b ? 2 : 1) * cell_bytes(bits, gs)));
+            if (cudaMalloc(&buf, count * (b ? 2 : 1) * cell_bytes(bits, gs)) != cudaSuccess) {   // no room for a copy: the launch chain
+                cudaGetLastError();
+                return FFAI_OK;
+            }
             L->owned_weights.push_back(buf);
             if (launch_retile_cells(a, b, static_cast<uint8_t*>(buf), n, N, K, bits, gs)) return fail(L, FFAI_ERR_CUDA, "re-tiling the experts failed");
             *out = static_cast<const uint8_t*>(buf);
