@@ -350,6 +350,26 @@ int launch_router_batched(const RouterParams& p, const uint16_t* x, int T, uint3
     // hidden axis into ranges of chunks as well and leave the ordered sum of the chunks to the routing kernel.
     if ((p.kind == FFAI_LINEAR_F32 || p.kind == FFAI_LINEAR_BF16) && p.hidden % 64 == 0 && T >= 256) {
         const int tiles = ((T + RB_TOK - 1) / RB_TOK) * ((p.n_experts + RB_EXP - 1) / RB_EXP);
+        // Twice as wide tiles, one block per SM, from the batch on that gives more than half of the SMs one (below that the
+        // narrow tiles, one per SM, take less); a last column of at most 64 experts would leave half a wide tile empty.
+        const int wide = tiles / 2;
+        if (((p.n_experts + RB_EXP - 1) / RB_EXP) % 2 == 0 && wide * 2 > n_sms) {
+            const dim3 grid((T + RB_TOK - 1) / RB_TOK, (p.n_experts + RW_EXP - 1) / RW_EXP);
+            static SmemOptIn opt1, opt2;
+            bool ok;
+            if (p.kind == FFAI_LINEAR_F32) {
+                ok = opt1.ensure(router_logits_wide_kernel<1>, RW_SMEM);
+                if (ok) router_logits_wide_kernel<1><<<grid, 256, RW_SMEM, st>>>(p, x, T, logits);
+            } else {
+                ok = opt2.ensure(router_logits_wide_kernel<2>, RW_SMEM);
+                if (ok) router_logits_wide_kernel<2><<<grid, 256, RW_SMEM, st>>>(p, x, T, logits);
+            }
+            if (ok) {
+                const int warps = 4;
+                route_only_kernel<<<(T + warps - 1) / warps, warps * 32, (size_t)warps * 2 * p.n_experts * sizeof(float), st>>>(p, logits, T, idx, w);
+                return cudaGetLastError() == cudaSuccess ? 2 : -1;
+            }
+        }
         int z = 1, per = n_chunks;
         float* part = nullptr;
         // measured at 256 experts: 128 tiles take 156 us un-split (one block per SM) against 169 us split three ways
