@@ -1982,7 +1982,7 @@ int forward_device(ffai_moe_layer* L, const uint16_t* x, int T, uint16_t* out, c
             tile_schedule_kernel<<<1, 32, 0, st>>>(L->offsets, E, tc_group_rows(L), L->tile_offsets);
             L->launches += 1;
         }
-        gather_rows_perm8_kernel<<<(M + 7) / 8, 256, 0, st>>>(x, L->perm, K, L->xg, M, H);
+        scatter_rows_perm8_kernel<<<T, 256, 0, st>>>(x, L->inv_perm, K, L->xg, H);
         L->launches += 1;
         stage_end(L, ST_GATHER, st);
 
