@@ -191,7 +191,13 @@ FFAI_DEVINL void route_token_warp(const RouterParams& p, float* logits_s, float*
         for (int e = lane; e < E; e += 32) logits_s[e] = __fmul_rn(logits_s[e], p.logit_scale);
         __syncwarp();
     }
-    if (p.gating_mode == 2) {
+    const bool sigmoid = p.gating_mode == 2;
+    const bool fast = (p.gating_mode == 1) ||
+                      (p.gating_mode == 0 && p.norm_topk_prob && p.expert_bias == nullptr);
+    // what the selection compares; the top-k itself appears once (three inlined copies cost the small-batch router 2 us in
+    // instruction fetches)
+    const float* by = scratch;
+    if (sigmoid) {
         // NemotronH routing (NemotronHText.swift:844-867): sigmoid scores; selection on score + bias; weights are the
         // raw sigmoids of the selected, over (their sum + 1e-20) when k > 1 and renormalising, times the scaling factor
         for (int e = lane; e < E; e += 32) {
@@ -199,9 +205,32 @@ FFAI_DEVINL void route_token_warp(const RouterParams& p, float* logits_s, float*
             logits_s[e] = sg;
             scratch[e] = p.expert_bias ? __fadd_rn(sg, p.expert_bias[e]) : sg;
         }
+    } else if (fast) {
+        // top-k of the logits, softmax over the picked (MoELayer.swift:146-172, 197-203)
+        by = logits_s;
+    } else {
+        // general softmax-then-top-k (MoELayer.swift:174-195)
+        float vmax = -INFINITY;
+        for (int e = lane; e < E; e += 32) vmax = fmaxf(vmax, logits_s[e]);
+#pragma unroll
+        for (int m = 16; m > 0; m >>= 1) vmax = fmaxf(vmax, __shfl_xor_sync(0xFFFFFFFFu, vmax, m));
+        for (int e = lane; e < E; e += 32) scratch[e] = det_expf(__fsub_rn(logits_s[e], vmax));
         __syncwarp();
-        warp_topk(scratch, E, K, lane, my_idx, my_val);
-        float w = (lane < K) ? logits_s[my_idx] : 0.0f;
+        float sum = 0.0f;
+        for (int e = 0; e < E; ++e) sum = __fadd_rn(sum, scratch[e]);  // ascending order, every lane
+        __syncwarp();
+        const bool degenerate = !(sum > 0.0f);
+        for (int e = lane; e < E; e += 32) {
+            float g = degenerate ? __fdiv_rn(1.0f, (float)E) : __fdiv_rn(scratch[e], sum);
+            if (p.expert_bias) g = __fadd_rn(g, p.expert_bias[e]);
+            scratch[e] = g;
+        }
+    }
+    __syncwarp();
+    warp_topk(by, E, K, lane, my_idx, my_val);
+    float w;
+    if (sigmoid) {
+        w = (lane < K) ? logits_s[my_idx] : 0.0f;
         if (K > 1 && p.norm_topk_prob) {
             float sum = 0.0f;
             for (int j = 0; j < K; ++j) sum = __fadd_rn(sum, __shfl_sync(0xFFFFFFFFu, w, j));
@@ -209,46 +238,19 @@ FFAI_DEVINL void route_token_warp(const RouterParams& p, float* logits_s, float*
             w = __fdiv_rn(w, sum);
         }
         w = __fmul_rn(w, p.routed_scaling);
-        if (p.per_expert_scale && lane < K) w = __fmul_rn(w, p.per_expert_scale[my_idx]);
-        if (lane < K) { idx_out[lane] = (uint32_t)my_idx; w_out[lane] = w; }
-        return;
-    }
-    const bool fast = (p.gating_mode == 1) ||
-                      (p.gating_mode == 0 && p.norm_topk_prob && p.expert_bias == nullptr);
-    if (fast) {
-        // top-k of the logits, softmax over the picked (MoELayer.swift:146-172, 197-203)
-        warp_topk(logits_s, E, K, lane, my_idx, my_val);
+    } else if (fast) {
         float vmax = __shfl_sync(0xFFFFFFFFu, my_val, 0);  // selection order is value-desc
         float ex = (lane < K) ? det_expf(__fsub_rn(my_val, vmax)) : 0.0f;
         float sum = 0.0f;
         for (int j = 0; j < K; ++j) sum = __fadd_rn(sum, __shfl_sync(0xFFFFFFFFu, ex, j));
-        float w = (sum > 0.0f) ? __fdiv_rn(ex, sum) : __fdiv_rn(1.0f, (float)K);
-        if (p.per_expert_scale && lane < K) w = __fmul_rn(w, p.per_expert_scale[my_idx]);
-        if (lane < K) { idx_out[lane] = (uint32_t)my_idx; w_out[lane] = w; }
-        return;
-    }
-    // general softmax-then-top-k (MoELayer.swift:174-195)
-    float vmax = -INFINITY;
-    for (int e = lane; e < E; e += 32) vmax = fmaxf(vmax, logits_s[e]);
-#pragma unroll
-    for (int m = 16; m > 0; m >>= 1) vmax = fmaxf(vmax, __shfl_xor_sync(0xFFFFFFFFu, vmax, m));
-    for (int e = lane; e < E; e += 32) scratch[e] = det_expf(__fsub_rn(logits_s[e], vmax));
-    __syncwarp();
-    float sum = 0.0f;
-    for (int e = 0; e < E; ++e) sum = __fadd_rn(sum, scratch[e]);  // ascending order, every lane
-    const bool degenerate = !(sum > 0.0f);
-    for (int e = lane; e < E; e += 32) {
-        float g = degenerate ? __fdiv_rn(1.0f, (float)E) : __fdiv_rn(scratch[e], sum);
-        if (p.expert_bias) g = __fadd_rn(g, p.expert_bias[e]);
-        scratch[e] = g;
-    }
-    __syncwarp();
-    warp_topk(scratch, E, K, lane, my_idx, my_val);
-    float w = my_val;
-    if (p.norm_topk_prob) {
-        float s2 = 0.0f;
-        for (int j = 0; j < K; ++j) s2 = __fadd_rn(s2, __shfl_sync(0xFFFFFFFFu, my_val, j));
-        if (s2 > 0.0f) w = __fdiv_rn(my_val, s2);
+        w = (sum > 0.0f) ? __fdiv_rn(ex, sum) : __fdiv_rn(1.0f, (float)K);
+    } else {
+        w = my_val;
+        if (p.norm_topk_prob) {
+            float s2 = 0.0f;
+            for (int j = 0; j < K; ++j) s2 = __fadd_rn(s2, __shfl_sync(0xFFFFFFFFu, my_val, j));
+            if (s2 > 0.0f) w = __fdiv_rn(my_val, s2);
+        }
     }
     if (p.per_expert_scale && lane < K) w = __fmul_rn(w, p.per_expert_scale[my_idx]);
     if (lane < K) { idx_out[lane] = (uint32_t)my_idx; w_out[lane] = w; }
