@@ -1462,14 +1462,20 @@ int ep_all_to_all(ffai_moe_layer* L, const uint8_t* send, const size_t* off_s, c
 int tc_group_rows(const ffai_moe_layer*) { return g100::BM; }
 bool tc_reads_cache(const ffai_moe_layer* L) { return L->exp_wbf[0] && (L->opt_tc_weights != 1 || L->cfg.expert_bits != 4); }
 bool tc_possible(const ffai_moe_layer* L) { return L->tc_ok && (L->cfg.expert_bits == 4 || L->exp_wbf[0]); }
-// Gate/up with few rows per expert goes over the packed weights even when the layer keeps a cache: an expert
-// then has one or two token tiles, the dequant stage runs once or twice per weight tile, and the 4x smaller
-// weight read wins (cfg3: 160 us packed against 170 us cached; at 256 rows per expert the cache wins, 300
-// against 339 us).  Down keeps the cache: its reduction axis is short and the packed pipeline's start-up per
-// item weighs more.
+// Few rows per expert go over the packed weights even when the layer keeps a cache: while most experts have one token
+// tile, the dequant stage runs once per weight tile and the 4x smaller weight read wins; from two tiles on the cache
+// does.  Packed against cached, us:
+//   32 experts of 2880, 97 rows each    gate/up 142 / 179   down  88 / 103     175 rows   263 / 242   160 / 148
+//   128 experts of 2048 x 768, 94 rows          121 / 152         68 /  78     128 rows   158 / 163    99 /  91
+//   256 experts of 2048 x 512, 62 rows          142 / 192         84 /  99     125 rows   195 / 211   125 / 115
+// Half of the experts have a second tile at 128 rows; down's short reduction axis pays for the packed pipeline's start-up
+// per item, so its line lies where second tiles begin.  Groups of 32 (two re-tiled scale words per block instead of one)
+// have it at the same place: 2880, 97 rows 152 / 183 and 97 / 109; 125 rows 199 / 209 and 121 / 123; 175 rows 277 / 252.
+bool packed_pays(const ffai_moe_layer* L, double rows_per_expert, double most) {
+    return L->cfg.expert_bits == 4 && L->opt_tc_weights == 0 && rows_per_expert <= most;
+}
 int tc_gate_up(ffai_moe_layer* L, const g100::Params& p, double rows_per_expert, cudaStream_t st) {
-    const bool packed_pays = L->cfg.expert_bits == 4 && L->opt_tc_weights == 0 && rows_per_expert <= 160.0;
-    if (tc_reads_cache(L) && !packed_pays) {
+    if (tc_reads_cache(L) && !packed_pays(L, rows_per_expert, 136.0)) {
         g100::Params pc = p;
         pc.wcache = L->exp_wbf[0]; pc.wcache2 = L->exp_wbf[1]; pc.cache_blocks = cache_blocks(p.n_out, true);
         return g100::launch_grouped_gemm<true, uint16_t, true>(L->tm_xg, L->tm_xg, L->tm_xg, pc, L->n_sms, st);
@@ -1477,8 +1483,8 @@ int tc_gate_up(ffai_moe_layer* L, const g100::Params& p, double rows_per_expert,
     return g100::launch_grouped_gemm<true, uint16_t>(L->tm_gate, L->tm_up, L->tm_xg, p, L->n_sms, st);
 }
 template <typename TOut>
-int tc_down(ffai_moe_layer* L, const g100::Params& p, cudaStream_t st) {
-    if (tc_reads_cache(L)) {
+int tc_down(ffai_moe_layer* L, const g100::Params& p, double rows_per_expert, cudaStream_t st) {
+    if (tc_reads_cache(L) && !packed_pays(L, rows_per_expert, 112.0)) {
         g100::Params pc = p;
         pc.wcache = L->exp_wbf[2]; pc.wcache2 = nullptr; pc.cache_blocks = cache_blocks(p.n_out, false);
         return g100::launch_grouped_gemm<false, TOut, true>(L->tm_inner, L->tm_inner, L->tm_inner, pc, L->n_sms, st);
@@ -1552,7 +1558,7 @@ int run_experts_on_rows(ffai_moe_layer* L, int n_rows, int n_exp, const uint32_t
         stage_begin(L, ST_GATE_UP, st);
         p.scales = L->w.gate_proj.scales; p.biases = L->w.gate_proj.biases; p.row_bias = L->w.gate_proj.row_bias;
         p.scales2 = L->w.up_proj.scales; p.biases2 = L->w.up_proj.biases; p.row_bias2 = L->w.up_proj.row_bias;
-        if (c.expert_group_size != 32) { p.sb = L->sb_gate; p.sb2 = L->sb_up; }
+        p.sb = L->sb_gate; p.sb2 = L->sb_up;
         p.n_out = I; p.K = H; p.m_tiles = (I + BN / 2 - 1) / (BN / 2);
         p.out = L->inner_bf; p.out_ld = I; p.out_permute8 = 1;
         if (tc_gate_up(L, p, rpe, st))
@@ -1561,11 +1567,11 @@ int run_experts_on_rows(ffai_moe_layer* L, int n_rows, int n_exp, const uint32_t
         stage_begin(L, ST_DOWN, st);
         p.scales = L->w.down_proj.scales; p.biases = L->w.down_proj.biases; p.row_bias = L->w.down_proj.row_bias;
         p.scales2 = nullptr; p.biases2 = nullptr; p.row_bias2 = nullptr;
-        p.sb = c.expert_group_size != 32 ? L->sb_down : nullptr; p.sb2 = nullptr;
+        p.sb = L->sb_down; p.sb2 = nullptr;
         p.n_out = H; p.K = I; p.m_tiles = (H + BN - 1) / BN;
         p.out = L->y; p.out_ld = H; p.out_permute8 = 0;
         if (L->ep_peer_on) p.out = L->ep_y_bf;
-        if (L->ep_peer_on ? tc_down<uint16_t>(L, p, st) : tc_down<float>(L, p, st))
+        if (L->ep_peer_on ? tc_down<uint16_t>(L, p, rpe, st) : tc_down<float>(L, p, rpe, st))
             return fail(L, FFAI_ERR_CUDA, "down grouped GEMM launch failed");
         stage_end(L, ST_DOWN, st);
         L->launches += 3;
@@ -1997,7 +2003,7 @@ int forward_device(ffai_moe_layer* L, const uint16_t* x, int T, uint16_t* out, c
         stage_begin(L, ST_GATE_UP, st);
         p.scales = L->w.gate_proj.scales; p.biases = L->w.gate_proj.biases; p.row_bias = L->w.gate_proj.row_bias;
         p.scales2 = L->w.up_proj.scales; p.biases2 = L->w.up_proj.biases; p.row_bias2 = L->w.up_proj.row_bias;
-        if (c.expert_group_size != 32) { p.sb = L->sb_gate; p.sb2 = L->sb_up; }
+        p.sb = L->sb_gate; p.sb2 = L->sb_up;
         p.n_out = I; p.K = H; p.m_tiles = (I + BN / 2 - 1) / (BN / 2);
         p.out = L->inner_bf; p.out_ld = I; p.out_permute8 = 1;
         if (tc_gate_up(L, p, rows_per_expert, st))
@@ -2009,10 +2015,10 @@ int forward_device(ffai_moe_layer* L, const uint16_t* x, int T, uint16_t* out, c
         p.timeline = nullptr;
         p.scales = L->w.down_proj.scales; p.biases = L->w.down_proj.biases; p.row_bias = L->w.down_proj.row_bias;
         p.scales2 = nullptr; p.biases2 = nullptr; p.row_bias2 = nullptr;
-        p.sb = c.expert_group_size != 32 ? L->sb_down : nullptr; p.sb2 = nullptr;
+        p.sb = L->sb_down; p.sb2 = nullptr;
         p.n_out = H; p.K = I; p.m_tiles = (H + BN - 1) / BN;
         p.out = L->y_bf; p.out_ld = H; p.out_permute8 = 0;
-        if (tc_down<uint16_t>(L, p, st))
+        if (tc_down<uint16_t>(L, p, rows_per_expert, st))
             return fail(L, FFAI_ERR_CUDA, "down grouped GEMM launch failed: %s", cudaGetErrorString(cudaGetLastError()));
         L->launches += 1;
         stage_end(L, ST_DOWN, st);

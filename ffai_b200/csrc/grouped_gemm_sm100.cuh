@@ -72,7 +72,7 @@ struct Params {
     const uint16_t* wcache;    // WBF16: the projection's tile-major bf16 cache, [E, cache_blocks, K/64] tiles of 16 KB
     const uint16_t* wcache2;   // WBF16, fused gate/up: the up projection's cache
     int cache_blocks;          // 128-row blocks per expert in a cache
-    const uint32_t* sb;        // nullable: (scale | bias << 16) words re-tiled [E, n_out/16, K/64, 16] (group 64 or 128)
+    const uint32_t* sb;        // nullable: (scale | bias << 16) words re-tiled [E, n_out/16, K/64, 16] (group 32: K/32)
     const uint32_t* sb2;
     int n_out;                 // output rows per expert
     int K;
@@ -566,6 +566,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
         const int r = (dw & 7) * 32 + lane;                         // 0..255
         const int gpr = p.K / p.group_size;
         const int gshift = p.group_size == 32 ? 5 : (p.group_size == 64 ? 6 : 7);
+        const int sw_shift = p.group_size == 32 ? 1 : 0;            // re-tiled words per 64-k block: two or one
         const bool second = FUSED && r >= BN / 2;                   // the up projection's half of the tile
         const uint16_t* sbase_ptr = second ? p.scales2 : p.scales;
         const uint16_t* bbase_ptr = second ? p.biases2 : p.biases;
@@ -598,7 +599,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
             RowScales rs;
             rs.sp = sbase_ptr + grow * gpr;
             rs.bq = bbase_ptr + grow * gpr;
-            rs.sw = sbw_ptr ? sbw_ptr + (((size_t)c.expert * (p.n_out >> 4) + (prow >> 4)) * KB) * 16 + (prow & 15) : nullptr;
+            rs.sw = sbw_ptr ? sbw_ptr + ((((size_t)c.expert * (p.n_out >> 4) + (prow >> 4)) * KB) << sw_shift) * 16 + (prow & 15) : nullptr;
             rs.j0 = (int)((grp ^ blocks_before_item) & 1u);
             return rs;
         };
@@ -611,8 +612,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
             for (int jj = 0; jj < 2; ++jj) {
                 const int kb = min(kb0 + rs.j0 + 2 * jj, KB - 1);
                 if (rs.sw) {
-                    nxt[jj][0] = __ldg(rs.sw + (size_t)kb * 16);
-                    nxt[jj][1] = nxt[jj][0];
+                    const uint32_t* w = rs.sw + ((size_t)kb << sw_shift) * 16;
+                    nxt[jj][0] = __ldg(w);
+                    nxt[jj][1] = __ldg(w + sw_shift * 16);
                 } else {
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {

@@ -296,8 +296,9 @@ FFAI_API uint32_t ffai_ep_plan_exchange(const uint32_t* recv_counts, int32_t wor
  *   "path"         0 automatic, 1 CUDA-core grouped GEMV only, 2 tcgen05 grouped GEMM whenever possible,
  *                  3 streaming decode kernels whenever possible
  *   "tc_min_rows"  smallest T*k that takes the tcgen05 path under "path" = 0 (0: default)
- *   "tc_weights"   tcgen05 path reads 0 automatic (the bf16 weight cache when the layer keeps one, except gate/up
- *                  with at most 160 routed rows per expert), 1 always the packed weights, 2 always the cache
+ *   "tc_weights"   tcgen05 path reads 0 automatic (the bf16 weight cache when the layer keeps one, except 4-bit experts
+ *                  with few rows each: gate/up to 136, down to 112), 1 always the packed weights (4-bit only),
+ *                  2 always the cache
  *   "host_chunks"  host entry points: 0 = a batch of 4096 tokens or more goes through in up to 3 chunks whose copies
  *                  overlap the compute (same bits: tokens are independent), 1 = always as one piece, 2..4 = at
  *                  most that many chunks
