@@ -541,3 +541,23 @@ def test_wide_router_tiles(oracle_mod, kind, T, E, H):
     mask = np.zeros(T, dtype=np.uint8)
     mask[:: 97] = 1     # routing is compared for every token, outputs for a sample
     run_and_check(oracle_mod, spec, T, token_mask=mask)
+
+
+# ── groups of 32 on the tensor-core path: the re-tiled scale words, two per 64-k block ──
+
+@pytest.mark.parametrize("H,I,T", [(320, 256, 130), (2880, 448, 45)])   # 5 / 45 and 4 / 7 blocks of 64: a last packed box of one, three and four blocks
+def test_tc_group32_packed_words(oracle_mod, H, I, T):
+    spec = synth.LayerSpec("tc_group32", H, I, 6, 3, expert_group_size=32, expert_row_bias=1, prefill_weight_cache=2)
+    host = synth.make_layer(spec, 5)
+    x = synth.make_tokens(T, H, 5)
+    layer = MoELayer(host, T)
+    try:
+        layer.set_option("path", TC)
+        layer.set_option("tc_weights", 2)
+        cached, _ = layer.forward_host(x)
+        layer.set_option("tc_weights", 1)
+        packed, _ = layer.forward_host(x)
+    finally:
+        layer.close()
+    assert np.array_equal(cached, packed)   # both round fma(q, scale, bias) to bf16 once and run the same MMA sequence
+    run_and_check(oracle_mod, spec, T, seed=5, host=host, path=TC, options={"tc_weights": 1})
