@@ -24,7 +24,9 @@
 // 16 x 64 cell).  Measured against the launch chain: 32 experts of 2880 x 2880, top 4: one token 42.7 -> 30.8 us, eight
 // tokens of group 32 111 -> 92; 128 experts of 2048 x 768, top 8, one token 41.8 -> 22; 8-bit codes, four tokens
 // 192 -> 50; 256 experts and a shared one, three tokens 102 -> 33.
-// fp32 accumulation throughout; only the activation's result is rounded to bf16, as in the launch chain.
+// fp32 accumulation throughout.  The activation's result is held as the launch chain holds it: rounded to bf16 for 4-bit
+// routed experts, in fp32 for 8-bit ones and for the shared expert.  The MMA reads the latter as three bf16 terms whose sum is
+// the fp32 value (split3): three times the MMAs of down, no bit lost.
 //
 // The waits at the grid barriers are bounded; a CTA that gives up raises the error word and leaves.
 #pragma once
@@ -82,8 +84,9 @@ struct Params {
     uint32_t* indices;          // [T, k]
     float* rweights;            // [T, k]
     PlanOut plan;
-    uint16_t* inner;            // [T*k, I] bf16, 8-run permuted
-    uint16_t* sh_inner;         // [T, Is]
+    uint16_t* inner;            // [INNER_TERMS planes][T*k, I] bf16, 8-run permuted
+    uint16_t* sh_inner;         // [3 planes][T, Is]
+    size_t inner_plane, sh_plane;   // elements between planes
     const uint16_t* residual;   // nullable
     uint16_t* out;
     float* split;               // [2 * CTAs][16 * MAX_T] partial sums of down items that two or more CTAs share
@@ -197,27 +200,50 @@ FFAI_DEVINL void a_fragment(const Raw<BITS, G32>& r, int w, int hp, uint32_t mas
     }
 }
 
+// Terms of an activation result: 1 = rounded to bf16, 3 = fp32 as a sum of bf16 values.
+template <int BITS>
+constexpr int INNER_TERMS = BITS == 8 ? 3 : 1;
+constexpr int SH_TERMS = 3;
+
+// v as three bf16 values whose sum is v: 24 significant bits are cut into 8 + 8 + 8 (the last ones are lost below 2^-133, the
+// smallest bf16).  Infinities and NaN stay in the first.
+FFAI_DEVINL void split3(float v, uint16_t (&term)[3]) {
+    const uint32_t b = __float_as_uint(v);
+    term[0] = (uint16_t)(b >> 16);
+    term[1] = term[2] = 0;
+    if ((b & 0x7F800000u) == 0x7F800000u) {
+        if (b & 0x007FFFFFu) term[0] |= 0x40;   // a NaN whose payload lies in the bits cut off
+        return;
+    }
+    const float r1 = __fsub_rn(v, __uint_as_float(b & 0xFFFF0000u));
+    const uint32_t m = __float_as_uint(r1);
+    term[1] = (uint16_t)(m >> 16);
+    term[2] = (uint16_t)(__float_as_uint(__fsub_rn(r1, __uint_as_float(m & 0xFFFF0000u))) >> 16);
+}
+
 // Sums over the 64 k (group 32: over each half) of the activation columns 2t and 2t+1: an MMA with a matrix of ones.
-template <bool G32>
-FFAI_DEVINL void column_sums(const uint4& x0, const uint4& x1, float (*sx)[2]) {
-    const uint32_t xb[2][4] = {{x0.x, x0.y, x0.z, x0.w}, {x1.x, x1.y, x1.z, x1.w}};
+template <bool G32, int TERMS>
+FFAI_DEVINL void column_sums(const uint4* x0, const uint4* x1, float (*sx)[2]) {
     const uint32_t ones[4] = {0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u};
     float c[4];
 #pragma unroll
     for (int w = 0; w < 2; ++w) {
-        if (G32 || w == 0) mma16816_zero(c, ones, xb[w][0], xb[w][1]);
-        else mma16816(c, ones, xb[w][0], xb[w][1]);
-        mma16816(c, ones, xb[w][2], xb[w][3]);
+#pragma unroll
+        for (int i = TERMS - 1; i >= 0; --i) {
+            const uint4& x = w ? x1[i] : x0[i];
+            if ((G32 || w == 0) && i == TERMS - 1) mma16816_zero(c, ones, x.x, x.y);
+            else mma16816(c, ones, x.x, x.y);
+            mma16816(c, ones, x.z, x.w);
+        }
         sx[G32 ? w : 0][0] = c[0]; sx[G32 ? w : 0][1] = c[1];
     }
 }
 
 // Adds the cell's contribution to rows g, g+8 (tot[0..1], tot[2..3]) and columns 2t, 2t+1, times the columns' weights
-// with WEIGHTED.  sx[half][column]: run sums.
-template <int BITS, bool G32, bool WEIGHTED>
-FFAI_DEVINL void cell_dot(const Raw<BITS, G32>& r, uint32_t mask, uint32_t expo, const uint4& x0, const uint4& x1, const float (*sx)[2], float w0,
+// with WEIGHTED.  x0, x1: the TERMS terms of the activations; sx[half][column]: run sums.
+template <int BITS, bool G32, bool WEIGHTED, int TERMS>
+FFAI_DEVINL void cell_dot(const Raw<BITS, G32>& r, uint32_t mask, uint32_t expo, const uint4* x0, const uint4* x1, const float (*sx)[2], float w0,
                           float w1, float* tot) {
-    const uint32_t xb[2][4] = {{x0.x, x0.y, x0.z, x0.w}, {x1.x, x1.y, x1.z, x1.w}};
     float c[2][4];
 #pragma unroll
     for (int w = 0; w < 2; ++w)
@@ -225,9 +251,13 @@ FFAI_DEVINL void cell_dot(const Raw<BITS, G32>& r, uint32_t mask, uint32_t expo,
         for (int hp = 0; hp < 2; ++hp) {
             uint32_t a[4];
             a_fragment<BITS, G32>(r, w, hp, mask, expo, a);
-            float* acc = c[G32 ? w : 0];
-            if ((G32 || w == 0) && hp == 0) mma16816_zero(acc, a, xb[w][0], xb[w][1]);
-            else mma16816(acc, a, xb[w][2 * hp], xb[w][2 * hp + 1]);
+#pragma unroll
+            for (int i = TERMS - 1; i >= 0; --i) {
+                const uint4& x = w ? x1[i] : x0[i];
+                float* acc = c[G32 ? w : 0];
+                if ((G32 || w == 0) && hp == 0 && i == TERMS - 1) mma16816_zero(acc, a, x.x, x.y);
+                else mma16816(acc, a, hp ? x.z : x.x, hp ? x.w : x.y);
+            }
         }
 #pragma unroll
     for (int h = 0; h < (G32 ? 2 : 1); ++h)
@@ -281,6 +311,7 @@ struct GateUp {
     int activation;
     float limit, alpha;
     uint16_t* inner;       // rows of I
+    size_t plane;          // elements between the terms of a result
 };
 
 // n cells cut into WARPS contiguous ranges: the first cell of a warp's range, and the warp whose range holds a cell.
@@ -293,7 +324,7 @@ FFAI_DEVINL int range_owner(int n, int cell) { return (int)((uint32_t)((cell + 1
 // warp + j (ranges are contiguous, so the slots are distinct and an item's are consecutive); after ONE __syncthreads per
 // batch the items are finished by all threads.  (With a __syncthreads per item and every warp on the same item an item
 // took 1.2 us at one token and 2.9 at eight, mostly waiting for the finishing warps.)
-template <int BITS, bool G32>
+template <int BITS, bool G32, int TERMS>
 FFAI_DEVINL void gate_up_phase(const GateUp& a, int T, int H, const Tables* tb, uint32_t x_u, int x_pitch, float* red,
                                int warp, int lane, uint32_t mask, uint32_t expo) {
     using C = Cell<BITS, G32>;
@@ -361,8 +392,8 @@ FFAI_DEVINL void gate_up_phase(const GateUp& a, int T, int H, const Tables* tb, 
             } else {
                 sx[0][0] = ld_s4(x0); sx[0][1] = ld_s4(x1);
             }
-            cell_dot<BITS, G32, false>(b.gate, mask, expo, xa, xb, sx, 0.0f, 0.0f, tot[0]);
-            cell_dot<BITS, G32, false>(b.up, mask, expo, xa, xb, sx, 0.0f, 0.0f, tot[1]);
+            cell_dot<BITS, G32, false, 1>(b.gate, mask, expo, &xa, &xb, sx, 0.0f, 0.0f, tot[0]);
+            cell_dot<BITS, G32, false, 1>(b.up, mask, expo, &xa, &xb, sx, 0.0f, 0.0f, tot[1]);
             fetch(b);
             xl += RUN; x0 += RUN; x1 += RUN;
             if (--here == 0) {
@@ -401,8 +432,16 @@ FFAI_DEVINL void gate_up_phase(const GateUp& a, int T, int H, const Tables* tb, 
                 const float* src = red + (size_t)(w0 + jj) * tile + col * RED_PITCH + r;
                 for (int w = w0; w <= w1; ++w, src += tile)
                     if (flat >= WARPS || range_begin(flat, w) < range_begin(flat, w + 1)) { sg += src[0]; su += src[T * RED_PITCH]; }
-                a.inner[(size_t)(tb->base[u] + col) * a.I + rb * 16 + dmma::permute8_col(r)] =
-                    f32_to_bf16_bits(glu_activation(sg, su, a.activation, a.limit, a.alpha));
+                const float v = glu_activation(sg, su, a.activation, a.limit, a.alpha);
+                uint16_t* to = a.inner + (size_t)(tb->base[u] + col) * a.I + rb * 16 + dmma::permute8_col(r);
+                if (TERMS == 1) {
+                    *to = f32_to_bf16_bits(v);
+                } else {
+                    uint16_t term[3];
+                    split3(v, term);
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) to[i * a.plane] = term[i];
+                }
             }
         }
         __syncthreads();   // the partial-sum slots are free
@@ -551,8 +590,8 @@ fused_decode_kernel(const Params p) {
             if (threadIdx.x == 0) { tb->expert[SHARED_U] = 0; tb->base[SHARED_U] = 0; tb->cnt[SHARED_U] = (uint16_t)T; }
         }
         __syncthreads();
-        const GateUp a{p.sh_gate_up, p.Is, SHARED_U, 1, nullptr, nullptr, 0, 0.0f, 0.0f, p.sh_inner};
-        gate_up_phase<SBITS == 0 ? 4 : SBITS, false>(a, T, H, tb, x_u, x_pitch, red, warp, lane, mask, expo);
+        const GateUp a{p.sh_gate_up, p.Is, SHARED_U, 1, nullptr, nullptr, 0, 0.0f, 0.0f, p.sh_inner, p.sh_plane};
+        gate_up_phase<SBITS == 0 ? 4 : SBITS, false, SH_TERMS>(a, T, H, tb, x_u, x_pitch, red, warp, lane, mask, expo);
     }
     if (!bar.wait(&tb->failed)) {
         if (threadIdx.x == 0) atomicExch(p.error_word, (uint32_t)ERR_GRID_BARRIER);
@@ -610,8 +649,8 @@ fused_decode_kernel(const Params p) {
 
     // ── phase 3: gate/up of the routed experts ──
     {
-        const GateUp a{p.gate_up, I, 0, U, p.rb_gate, p.rb_up, p.activation, p.limit, p.alpha, p.inner};
-        gate_up_phase<BITS, G32>(a, T, H, tb, x_u, x_pitch, red, warp, lane, mask, expo);
+        const GateUp a{p.gate_up, I, 0, U, p.rb_gate, p.rb_up, p.activation, p.limit, p.alpha, p.inner, p.inner_plane};
+        gate_up_phase<BITS, G32, INNER_TERMS<BITS>>(a, T, H, tb, x_u, x_pitch, red, warp, lane, mask, expo);
     }
 
     // ── phase 4: down over all experts of a 16-row block ──
@@ -681,20 +720,25 @@ fused_decode_kernel(const Params p) {
         using CC = std::conditional_t<SH, CS, C>;
         constexpr int B = SH ? (SBITS == 0 ? 4 : SBITS) : BITS;
         constexpr bool H32 = SH ? false : G32;
-        constexpr int AHEAD = CC::CELLS_AHEAD;
+        constexpr int TERMS = SH ? SH_TERMS : INNER_TERMS<BITS>;
+        constexpr int AHEAD = TERMS == 3 ? 2 : CC::CELLS_AHEAD;
+        const size_t plane = SH ? p.sh_plane : p.inner_plane;
         const int u = SH ? SHARED_U : w.u;
         const int row = tb->pos[u][g], ld = SH ? p.Is : I;
         const float w0 = tb->colw[u][2 * t], w1 = tb->colw[u][2 * t + 1];
         // columns without this expert: zero fragments and weight
         const uint16_t* xp = (SH ? p.sh_inner : p.inner) + (size_t)max(row, 0) * ld + w.c * 64 + (H32 ? 8 : 16) * t;
         const uint8_t *src_w = weights_at(w) + lane * 16, *src_s = weights_at(w) + CC::W + g * (H32 ? 16 : 8);
-        struct Ahead { Raw<B, H32> raw; uint4 x0, x1; } buf[AHEAD] = {};   // (columns without a row keep zeros)
+        struct Ahead { Raw<B, H32> raw; uint4 x0[TERMS], x1[TERMS]; } buf[AHEAD] = {};   // (columns without a row keep zeros)
         int p_n = n;
         auto fetch = [&](Ahead& d) {
             const bool on = p_n > 0;
             load_raw<B, H32>(on, src_w, src_s, d.raw);
-            ldcg16_if(on && row >= 0, xp, d.x0);
-            ldcg16_if(on && row >= 0, xp + (H32 ? 32 : 8), d.x1);
+#pragma unroll
+            for (int i = 0; i < TERMS; ++i) {
+                ldcg16_if(on && row >= 0, xp + i * plane, d.x0[i]);
+                ldcg16_if(on && row >= 0, xp + i * plane + (H32 ? 32 : 8), d.x1[i]);
+            }
             src_w += CC::BYTES; src_s += CC::BYTES; xp += 64; --p_n;
         };
 #pragma unroll
@@ -703,10 +747,9 @@ fused_decode_kernel(const Params p) {
         while (n > 0) {
 #pragma unroll
             for (int d = 0; d < AHEAD; ++d) {
-                const uint4 x0 = buf[d].x0, x1 = buf[d].x1;
                 float sx[2][2];
-                column_sums<H32>(x0, x1, sx);
-                cell_dot<B, H32, true>(buf[d].raw, mask, expo, x0, x1, sx, w0, w1, tot);
+                column_sums<H32, TERMS>(buf[d].x0, buf[d].x1, sx);
+                cell_dot<B, H32, true, TERMS>(buf[d].raw, mask, expo, buf[d].x0, buf[d].x1, sx, w0, w1, tot);
                 fetch(buf[d]);
                 if (--n == 0) break;
             }

@@ -87,8 +87,8 @@ struct ffai_moe_layer {
     const uint8_t* fd_sh_gate_up = nullptr;  // ... and of the shared expert
     const uint8_t* fd_sh_down = nullptr;
     const float* fd_sh_gate_f32 = nullptr;   // a quantized shared-expert gate expanded to fp32
-    uint16_t* fd_inner = nullptr;            // [fdec::MAX_ROWS, I] activation results
-    uint16_t* fd_sh_inner = nullptr;         // [fdec::MAX_T, Is]
+    uint16_t* fd_inner = nullptr;            // [terms][fdec::MAX_ROWS, I] activation results
+    uint16_t* fd_sh_inner = nullptr;         // [terms][fdec::MAX_T, Is]
     float* fd_split = nullptr;               // [2 * SMs][16 * fdec::MAX_T]
     uint32_t* fd_sync = nullptr;             // grid barrier word, then one ticket per 16-row block of the output (self-resetting)
     int opt_decode = 0;              // decode kernels: 0 automatic, 1 per-lane cp.async rings, 2 bulk-copy streams
@@ -914,8 +914,9 @@ extern "C" FFAI_API int ffai_moe_create(const ffai_moe_config* config, ffai_moe_
     L->fused_planned = world == 1 && cc_major == 10 && !L->no_gate && (c.expert_bits == 4 || c.expert_bits == 8) &&
                        (c.shared_intermediate == 0 || ((c.shared_bits == 4 || c.shared_bits == 8) && c.shared_group_size != 32));
     if (L->fused_planned) {
-        if ((rc = ws_alloc(L, &L->fd_inner, fdec::MAX_ROWS * I))) return rc;
-        if ((rc = ws_alloc(L, &L->fd_sh_inner, (size_t)fdec::MAX_T * c.shared_intermediate))) return rc;
+        const int terms = c.expert_bits == 8 ? fdec::INNER_TERMS<8> : fdec::INNER_TERMS<4>;
+        if ((rc = ws_alloc(L, &L->fd_inner, terms * fdec::MAX_ROWS * I))) return rc;
+        if ((rc = ws_alloc(L, &L->fd_sh_inner, (size_t)fdec::SH_TERMS * fdec::MAX_T * c.shared_intermediate))) return rc;
         if ((rc = ws_alloc(L, &L->fd_split, (size_t)2 * L->n_sms * 16 * fdec::MAX_T))) return rc;
         if ((rc = ws_alloc(L, &L->fd_sync, 1 + H / 16))) return rc;
         CUDA_TRY(L, cudaMemset(L->fd_sync, 0, (1 + H / 16) * 4));
@@ -1748,6 +1749,7 @@ int forward_device(ffai_moe_layer* L, const uint16_t* x, int T, uint16_t* out, c
         p.logits = L->logits; p.indices = L->indices; p.rweights = L->rweights;
         p.plan = PlanOut{L->counts, L->offsets, L->perm, L->inv_perm, nullptr};
         p.inner = L->fd_inner; p.sh_inner = L->fd_sh_inner;
+        p.inner_plane = (size_t)fdec::MAX_ROWS * I; p.sh_plane = (size_t)fdec::MAX_T * c.shared_intermediate;
         p.residual = residual; p.out = out;
         p.split = L->fd_split; p.barrier = L->fd_sync; p.tickets = L->fd_sync + 1; p.error_word = L->error_word;
         if (launch_fused_decode(p, c.expert_bits, c.expert_group_size == 32, c.shared_intermediate > 0 ? c.shared_bits : 0, L->n_sms, st)) {
