@@ -240,10 +240,11 @@ FFAI_DEVINL void column_sums(const uint4* x0, const uint4* x1, float (*sx)[2]) {
 }
 
 // Adds the cell's contribution to rows g, g+8 (tot[0..1], tot[2..3]) and columns 2t, 2t+1, times the columns' weights
-// with WEIGHTED.  x0, x1: the TERMS terms of the activations; sx[half][column]: run sums.
+// with WEIGHTED.  x0, x1: the TERMS terms of the activations; sx[half][column]: run sums.  WEIGHTED leaves a column whose token
+// does not have this expert (`on`) alone: its products are zero, but zero times an infinite scale is not.
 template <int BITS, bool G32, bool WEIGHTED, int TERMS>
 FFAI_DEVINL void cell_dot(const Raw<BITS, G32>& r, uint32_t mask, uint32_t expo, const uint4* x0, const uint4* x1, const float (*sx)[2], float w0,
-                          float w1, float* tot) {
+                          float w1, bool on0, bool on1, float* tot) {
     float c[2][4];
 #pragma unroll
     for (int w = 0; w < 2; ++w)
@@ -268,8 +269,10 @@ FFAI_DEVINL void cell_dot(const Raw<BITS, G32>& r, uint32_t mask, uint32_t expo,
 #pragma unroll
             for (int col = 0; col < 2; ++col) {
                 float& t = tot[2 * i + col];
-                if (WEIGHTED) t = fmaf(col ? w1 : w0, fmaf(bm, sx[h][col], sc * c[h][2 * i + col]), t);
-                else t = fmaf(bm, sx[h][col], fmaf(sc, c[h][2 * i + col], t));
+                if (WEIGHTED) {
+                    const float v = fmaf(col ? w1 : w0, fmaf(bm, sx[h][col], sc * c[h][2 * i + col]), t);
+                    if (col ? on1 : on0) t = v;
+                } else t = fmaf(bm, sx[h][col], fmaf(sc, c[h][2 * i + col], t));
             }
         }
 }
@@ -392,8 +395,8 @@ FFAI_DEVINL void gate_up_phase(const GateUp& a, int T, int H, const Tables* tb, 
             } else {
                 sx[0][0] = ld_s4(x0); sx[0][1] = ld_s4(x1);
             }
-            cell_dot<BITS, G32, false, 1>(b.gate, mask, expo, &xa, &xb, sx, 0.0f, 0.0f, tot[0]);
-            cell_dot<BITS, G32, false, 1>(b.up, mask, expo, &xa, &xb, sx, 0.0f, 0.0f, tot[1]);
+            cell_dot<BITS, G32, false, 1>(b.gate, mask, expo, &xa, &xb, sx, 0.0f, 0.0f, true, true, tot[0]);
+            cell_dot<BITS, G32, false, 1>(b.up, mask, expo, &xa, &xb, sx, 0.0f, 0.0f, true, true, tot[1]);
             fetch(b);
             xl += RUN; x0 += RUN; x1 += RUN;
             if (--here == 0) {
@@ -726,7 +729,8 @@ fused_decode_kernel(const Params p) {
         const int u = SH ? SHARED_U : w.u;
         const int row = tb->pos[u][g], ld = SH ? p.Is : I;
         const float w0 = tb->colw[u][2 * t], w1 = tb->colw[u][2 * t + 1];
-        // columns without this expert: zero fragments and weight
+        const bool on0 = tb->pos[u][2 * t] >= 0, on1 = tb->pos[u][2 * t + 1] >= 0;
+        // columns without this expert: zero fragments
         const uint16_t* xp = (SH ? p.sh_inner : p.inner) + (size_t)max(row, 0) * ld + w.c * 64 + (H32 ? 8 : 16) * t;
         const uint8_t *src_w = weights_at(w) + lane * 16, *src_s = weights_at(w) + CC::W + g * (H32 ? 16 : 8);
         struct Ahead { Raw<B, H32> raw; uint4 x0[TERMS], x1[TERMS]; } buf[AHEAD] = {};   // (columns without a row keep zeros)
@@ -749,7 +753,7 @@ fused_decode_kernel(const Params p) {
             for (int d = 0; d < AHEAD; ++d) {
                 float sx[2][2];
                 column_sums<H32, TERMS>(buf[d].x0, buf[d].x1, sx);
-                cell_dot<B, H32, true, TERMS>(buf[d].raw, mask, expo, buf[d].x0, buf[d].x1, sx, w0, w1, tot);
+                cell_dot<B, H32, true, TERMS>(buf[d].raw, mask, expo, buf[d].x0, buf[d].x1, sx, w0, w1, on0, on1, tot);
                 fetch(buf[d]);
                 if (--n == 0) break;
             }

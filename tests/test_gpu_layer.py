@@ -583,3 +583,26 @@ def test_one_launch_keeps_fp32_activation_results(oracle_mod, gs, shared_bits, T
     ref = oracle_mod.moe_forward(host, x)
     differ = float(np.mean(out != synth.f32_to_bf16(ref.out_f32)))
     assert differ <= 0.005, f"{100 * differ:.2f} % of the outputs differ from the rounded fp32 result"
+
+
+@pytest.mark.parametrize("bits,gs", [(4, 64), (4, 32), (8, 64)])
+@pytest.mark.parametrize("field,value", [("scales", np.inf), ("biases", np.nan)])
+def test_one_launch_confines_non_finite_weights(oracle_mod, bits, gs, field, value):
+    """An infinite or undefined scale of one expert reaches the tokens that selected it and no others."""
+    spec = synth.LayerSpec("non_finite", 512, 256, 16, 4, expert_bits=bits, expert_group_size=gs)
+    host = synth.make_layer(spec, 31)
+    x = synth.make_tokens(8, spec.hidden, 31)
+    ref = oracle_mod.moe_forward(host, x)
+    share = np.array([(ref.indices == e).any(axis=1).mean() for e in range(16)])
+    e = int(np.argmin(np.abs(share - 0.4)))             # some tokens select it, some do not
+    has = (ref.indices == e).any(axis=1)
+    assert has.any() and not has.all()
+    host.arrays["experts.down_proj." + field][e] = 0x7F80 if value == np.inf else 0x7FC0
+    layer = MoELayer(host, 8)
+    try:
+        out, dbg = layer.forward_host(x, debug=True)
+        assert layer.launch_count() == 1
+    finally:
+        layer.close()
+    assert np.array_equal(dbg.indices, ref.indices)
+    assert_parity(out[~has], ref.out_f32[~has], what=spec.name)
