@@ -16,14 +16,15 @@
 //   barrier  (the first weights of phase 4 are on their way into L2)
 //   phase 4  down: items of 16 output rows over ALL selected experts (and the shared one), each expert's product
 //            scaled by its combine weight, so the sum over warps is the block's output: no y buffer, no combine
-// Operands: 16 weight rows x 64 k per cell, re-tiled at load time in MMA fragment order (expert_stream_decode.cuh
-// describes the 4-bit cell), loaded straight into registers: every cell is used once, by one warp, so shared memory would
-// only add instructions (bulk copies into per-warp rings measured the same at one token and 10 % slower at eight).
+// Operands: cells of 16 weight rows x 64 k, loaded straight into registers: every cell is used once, by one warp, so shared
+// memory would only add instructions (bulk copies into per-warp rings measured the same at one token and 10 % slower at
+// eight).  4-bit experts of group 64 and 128 are read from the streams that expert_stream_decode.cuh keeps anyway; all others
+// from the packed rows as they are: no further copy of the experts.
 // mma.sync m16n8k16 has 8 columns: the tokens.  Bound: at one to four tokens latency (launch, two barriers, the cold
 // instruction fetches of code that runs once), at eight the issue slots of unpack and fold (about 105 instructions per
-// 16 x 64 cell).  Measured against the launch chain: 32 experts of 2880 x 2880, top 4: one token 42.7 -> 30.8 us, eight
-// tokens of group 32 111 -> 92; 128 experts of 2048 x 768, top 8, one token 41.8 -> 22; 8-bit codes, four tokens
-// 192 -> 50; 256 experts and a shared one, three tokens 102 -> 33.
+// 16 x 64 cell; packed rows 12 more than streams).  Measured against the launch chain: 32 experts of 2880 x 2880, top 4, one
+// token 42.7 -> 30.8 us, group 32, one token 47.1 -> 37.3, six 101 -> 92; 128 experts of 2048 x 768, top 8, one token
+// 41.8 -> 21; 8-bit codes, four tokens 196 -> 63; 256 experts and a shared one, three tokens 102 -> 37.
 // fp32 accumulation throughout.  The activation's result is held as the launch chain holds it: rounded to bf16 for 4-bit
 // routed experts, in fp32 for 8-bit ones and for the shared expert.  The MMA reads the latter as three bf16 terms whose sum is
 // the fp32 value (split3): three times the MMAs of down, no bit lost.
@@ -50,18 +51,24 @@ constexpr int MAX_DOWN_ITEMS = 12;             // down items a CTA's range may t
 constexpr uint32_t BARRIER_TRIES = 1u << 21;   // polls of about half a microsecond
 enum : uint32_t { ERR_GRID_BARRIER = 64 };
 
-// Cell: 16 weight rows x 64 k.  Words first (lane l's at l * 16, for 8-bit codes rows g+8 512 bytes further), then the
-// (scale | bias << 16) words of rows g and g+8, 8 bytes per g (group 32: both halves of the run, 16 bytes per g).
-// Lane (g, t) holds the 8-runs 2t and 2t+1 of the cell's k (group 32: runs t and t+4, so that a run's two MMAs stay in
-// one half).  8-bit: an 8-run is the bytes k0 k1 k4 k5 | k2 k3 k6 k7.
+// Where the weights of a cell lie.  STREAM: one run in MMA fragment order, words first (lane l's at l * 16), then the
+// (scale | bias << 16) words of rows g and g+8, 8 bytes per g.  ROWS: the packed rows, scales and biases as the layer has
+// them.  ROWS_SB: the packed rows, and the (scale | bias << 16) words re-tiled as [16-row block][32-run][16 rows].
+// Lane (g, t) holds the 8-runs 2t and 2t+1 of the cell's k in rows g and g+8 (group 32: runs t and t+4, so that a run's two
+// MMAs stay in one half).
+enum Source { STREAM, ROWS, ROWS_SB };
 template <int BITS, bool G32>
-struct Cell {
-    static constexpr int W = BITS == 4 ? 512 : 1024;
-    static constexpr int BYTES = W + (G32 ? 128 : 64);
-    // loads in flight per warp (1 in gate/up: 9.3 -> 11.4 us at one token of the 32-expert layer; 3 and 5: no gain, and the
-    // longer unrolled loop costs instruction fetches)
-    static constexpr int PAIRS_AHEAD = 2;   // gate/up: (gate cell, up cell) pairs
-    static constexpr int CELLS_AHEAD = 3;   // down
+constexpr Source SOURCE = BITS == 8 ? ROWS : (G32 ? ROWS_SB : STREAM);
+// loads in flight per warp (1 in gate/up: 9.3 -> 11.4 us at one token of the 32-expert layer; 3 and 5: no gain, and the
+// longer unrolled loop costs instruction fetches)
+constexpr int PAIRS_AHEAD = 2;   // gate/up: (gate cell, up cell) pairs
+constexpr int CELLS_AHEAD = 3;   // down (2 with activations of three terms)
+
+// One stacked projection.  STREAM: w alone (gate/up: gate and up cells of a 64-run alternate).
+struct Proj {
+    const uint8_t* w;
+    const uint8_t* s;   // scales (ROWS_SB: the re-tiled words)
+    const uint8_t* b;   // biases
 };
 
 struct Params {
@@ -69,16 +76,18 @@ struct Params {
     const uint16_t* x;          // [T, H]
     const uint16_t* xr;         // the router's rows (x unless split)
     int T, H, I;
-    const uint8_t* gate_up;     // routed streams
-    const uint8_t* down;
+    Proj gate, up, down;        // routed experts
+    int gshift;                 // log2 of the group size
     const uint16_t *rb_gate, *rb_up, *rb_down;   // nullable row biases
     int activation;
     float limit, alpha;
     int Is;                     // shared expert: 0 = none
-    const uint8_t* sh_gate_up;
-    const uint8_t* sh_down;
-    int sh_gate_kind;           // 0 none, 1 fp32, 2 bf16
+    Proj sh_gate, sh_up, sh_down;
+    int sh_gshift;
+    int sh_gate_kind;           // 0 none, 1 fp32, 2 bf16, 3 affine
     const void* sh_gate_w;      // [H]
+    const uint16_t *sh_gate_s, *sh_gate_b;
+    int sh_gate_bits, sh_gate_group;
     float* sh_gate_logit;       // [T]
     float* logits;              // [T, E]
     uint32_t* indices;          // [T, k]
@@ -86,7 +95,7 @@ struct Params {
     PlanOut plan;
     uint16_t* inner;            // [INNER_TERMS planes][T*k, I] bf16, 8-run permuted
     uint16_t* sh_inner;         // [3 planes][T, Is]
-    size_t inner_plane, sh_plane;   // elements between planes
+    uint32_t inner_plane, sh_plane;   // elements between planes
     const uint16_t* residual;   // nullable
     uint16_t* out;
     float* split;               // [2 * CTAs][16 * MAX_T] partial sums of down items that two or more CTAs share
@@ -112,6 +121,9 @@ struct Tables {
 // stride lets 8 threads read the same piece of 8 runs from distinct banks (router), the row pitch does so for the MMA
 // fragments of neighbouring rows.
 constexpr int RUN = 144, RUN_SUM = 128, RUN_HALF_SUMS = 136;
+// Gate/up items of a CTA whose partial sums fit the area at a time (a slot has 2 * T * RED_PITCH floats, an item up to WARPS slots).
+__host__ __device__ constexpr int gate_up_batch(int T) { return RED_BYTES / 4 / (2 * T * RED_PITCH) - (WARPS - 1); }
+
 template <int BITS, bool G32>
 struct Layout {
     static constexpr int STAGE_BYTES = 56 * 1024;
@@ -125,6 +137,11 @@ struct Layout {
     __host__ __device__ static int total(int T, int H) { return x() + T * x_pitch(H); }
     // the router's rows are staged in an area of their own, its chunk sums and the routing tables in the partial-sum area
     static bool fits(int T, int M, int E, int H, int I, int Is, int weight_bytes, int grid) {
+        if (SOURCE<BITS, G32> != STREAM && (double)E * H * I * BITS / 8 >= 4e9) return false;   // 32-bit byte offsets
+        // Packed rows of group 32 take 12 instructions a cell more than a stream; once a CTA's gate/up items need a second batch
+        // of partial sums, the launch chain is faster: 32 experts of 2880, 5 / 6 / 7 / 8 tokens 86 / 94 / 98 / 117 us here, 95 / 101 / 103 /
+        // 109 there (the eighth needs two); 128 experts of 2048 x 768, always one, 1 / 4 / 8 tokens 24 / 46 / 68 and 39 / 53 / 72.
+        if (SOURCE<BITS, G32> == ROWS_SB && (M < E ? M : E) * (I / 16) > gate_up_batch(T) * grid) return false;
         const int rows = (E + grid - 1) / grid;
         return rows * H * weight_bytes <= STAGE_BYTES && rows * T * (H / 64) * 4 <= RED_BYTES && T * 2 * E * 4 <= RED_BYTES &&
                H / 16 <= (MAX_DOWN_ITEMS - 2) * grid &&
@@ -145,11 +162,20 @@ FFAI_DEVINL void mma16816_zero(float* c, const uint32_t* a, uint32_t b0, uint32_
         : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.0f));
 }
 // A lane's part of a cell as it comes from memory.
-template <int BITS, bool G32>
+template <int BITS, bool G32, Source SRC>
 struct Raw {
-    uint4 w[BITS == 4 ? 1 : 2];
-    uint4 s4;   // scale words of rows g, g+8 (group 32: of the first half, then of the second)
-    FFAI_DEVINL uint32_t s(int h, int i) const { return h ? (i ? s4.w : s4.z) : (i ? s4.y : s4.x); }
+    uint4 w[BITS == 4 ? 1 : 2];            // 4 bits: rows g (x, y) and g+8 (z, w); 8 bits: row g, row g+8
+    uint32_t s[SRC == ROWS_SB ? 4 : 2];    // ROWS: scales of rows g, g+8 (group 32: both halves); else scale | bias << 16 ...
+    uint32_t b[2];                         // ROWS: biases
+    // of half h of the cell (group 32) and row half i
+    FFAI_DEVINL float scale(int h, int i) const {
+        if (SRC == ROWS) return __uint_as_float(G32 && h ? s[i] & 0xFFFF0000u : s[i] << 16);
+        return __uint_as_float(s[SRC == ROWS_SB ? 2 * h + i : i] << 16);
+    }
+    FFAI_DEVINL float bias(int h, int i) const {
+        if (SRC == ROWS) return __uint_as_float(G32 && h ? b[i] & 0xFFFF0000u : b[i] << 16);
+        return __uint_as_float(s[SRC == ROWS_SB ? 2 * h + i : i] & 0xFFFF0000u);
+    }
 };
 // Loads under a predicate, the registers keeping what they hold otherwise.  (With the load in a branch the compiler
 // loads into other registers and moves: the move waits for the load, and nothing is ahead any more.)
@@ -165,13 +191,101 @@ FFAI_DEVINL void ldcg16_if(bool on, const uint16_t* p, uint4& v) {   // written 
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %5, 0;\n\t@p ld.global.cg.v4.u32 {%0,%1,%2,%3}, [%4];\n\t}"
                  : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w) : "l"(p), "r"((int)on));
 }
-// `words` and `scales` are the lane's own addresses in the cell.
-template <int BITS, bool G32>
-FFAI_DEVINL void load_raw(bool on, const uint8_t* words, const uint8_t* scales, Raw<BITS, G32>& r) {
+// Pieces that do not fill a sector, or share it with the next cells': kept in L1.
+FFAI_DEVINL void ldg4_if(bool on, const uint8_t* p, uint32_t& v) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p ld.global.nc.u32 %0, [%1];\n\t}" : "+r"(v) : "l"(p), "r"((int)on));
+}
+FFAI_DEVINL void ldg2_if(bool on, const uint8_t* p, uint32_t& v) {
+    asm volatile("{\n\t.reg .pred p;\n\t.reg .u16 h;\n\tsetp.ne.b32 p, %2, 0;\n\t@p ld.global.nc.u16 h, [%1];\n\t@p cvt.u32.u16 %0, h;\n\t}"
+                 : "+r"(v) : "l"(p), "r"((int)on));
+}
+// Where a lane reads the cells of an item (16 rows of n_cells cells) from.  STREAM: addresses.  ROWS: 32-bit byte offsets into
+// a projection's words and scales (gate and up have the same shape, so the same ones), which an instruction adds to the
+// base by itself; `Layout::fits` keeps larger projections out.
+template <int BITS, bool G32, Source SRC>
+struct Cursor {
+    static constexpr int NB = BITS * 8;          // ROWS: bytes of a row per cell
+    uint32_t w, s, k;                            // k: of the cell (groups of 64 and 128)
+    // row block `rb` = expert * row blocks + row block of the expert; cell c
+    FFAI_DEVINL void seek(const Proj&, uint32_t rb, int n_cells, int c, int, int gshift, int lane) {
+        const uint32_t g = lane >> 2, t = lane & 3;
+        w = ((rb * 16 + g) * n_cells + c) * NB + t * (BITS == 8 ? (G32 ? 8 : 16) : (G32 ? 4 : 8));
+        if (SRC == ROWS_SB) s = ((rb * n_cells + c) * 32 + g) * 4;
+        else if (G32) s = ((rb * 16 + g) * n_cells + c) * 4;
+        else s = (rb * 16 + g) * ((uint32_t)(n_cells * 64) >> gshift) * 2;
+        k = c * 64;
+    }
+    FFAI_DEVINL void next(int) {
+        w += NB;
+        if (SRC == ROWS_SB) s += 128;
+        else if (G32) s += 4;
+        else k += 64;
+    }
+    FFAI_DEVINL void load(bool on, const Proj& p, int, int n_cells, int gshift, Raw<BITS, G32, SRC>& r) const {
+        const uint32_t w8 = w + (uint32_t)n_cells * NB * 8;
+        if (BITS == 8) {
+            uint4& far = r.w[1 % (BITS / 4)];
+            if (G32) {
+                ldg8_if(on, p.w + w, r.w[0].x, r.w[0].y); ldg8_if(on, p.w + w + 32, r.w[0].z, r.w[0].w);
+                ldg8_if(on, p.w + w8, far.x, far.y); ldg8_if(on, p.w + w8 + 32, far.z, far.w);
+            } else {
+                ldg16_if(on, p.w + w, r.w[0]); ldg16_if(on, p.w + w8, far);
+            }
+        } else if (G32) {
+            ldg4_if(on, p.w + w, r.w[0].x); ldg4_if(on, p.w + w + 16, r.w[0].y);
+            ldg4_if(on, p.w + w8, r.w[0].z); ldg4_if(on, p.w + w8 + 16, r.w[0].w);
+        } else {
+            ldg8_if(on, p.w + w, r.w[0].x, r.w[0].y); ldg8_if(on, p.w + w8, r.w[0].z, r.w[0].w);
+        }
+        if (SRC == ROWS_SB) {
 #pragma unroll
-    for (int i = 0; i < (BITS == 4 ? 1 : 2); ++i) ldg16_if(on, words + 512 * i, r.w[i]);
-    if (G32) ldg16_if(on, scales, r.s4);
-    else ldg8_if(on, scales, r.s4.x, r.s4.y);
+            for (int i = 0; i < 4; ++i) ldg4_if(on, p.s + s + 32 * i, r.s[i % (SRC == ROWS_SB ? 4 : 2)]);
+            return;
+        }
+        const uint32_t s0 = G32 ? s : s + (k >> gshift) * 2, s8 = s0 + ((uint32_t)(n_cells * 64) >> gshift) * 16;
+        if (G32) {
+            ldg4_if(on, p.s + s0, r.s[0]); ldg4_if(on, p.s + s8, r.s[1]); ldg4_if(on, p.b + s0, r.b[0]); ldg4_if(on, p.b + s8, r.b[1]);
+        } else {
+            ldg2_if(on, p.s + s0, r.s[0]); ldg2_if(on, p.s + s8, r.s[1]); ldg2_if(on, p.b + s0, r.b[0]); ldg2_if(on, p.b + s8, r.b[1]);
+        }
+    }
+};
+template <int BITS, bool G32>
+struct Cursor<BITS, G32, STREAM> {
+    static constexpr int CELL_BYTES = 576;
+    const uint8_t *w, *s;
+    FFAI_DEVINL void seek(const Proj& p, size_t rb, int n_cells, int c, int projections, int, int lane) {   // projections alternate
+        w = p.w + (rb * n_cells + c) * (CELL_BYTES * projections) + lane * 16;
+        s = p.w + (rb * n_cells + c) * (CELL_BYTES * projections) + 512 + (lane >> 2) * 8;
+    }
+    FFAI_DEVINL void next(int projections) { w += CELL_BYTES * projections; s += CELL_BYTES * projections; }
+    FFAI_DEVINL void load(bool on, const Proj&, int projection, int, int, Raw<BITS, G32, STREAM>& r) const {
+        ldg16_if(on, w + CELL_BYTES * projection, r.w[0]);
+        ldg8_if(on, s + CELL_BYTES * projection, r.s[0], r.s[1]);
+    }
+};
+// The first bytes (at most `budget`) of n cells of an item on their way into L2; returns the bytes asked for.
+template <int BITS, bool G32, Source SRC>
+FFAI_DEVINL int prefetch_cells(const Proj& p, size_t rb, int n_cells, int c, int n, int gshift, int budget, int lane) {
+    auto ask = [](const uint8_t* a) { asm volatile("prefetch.global.L2 [%0];" ::"l"(a)); };
+    if (SRC == STREAM) {
+        const int bytes = min(n * 576, budget);
+        for (int o = lane * 128; o < bytes; o += 32 * 128) ask(p.w + (rb * n_cells + c) * 576 + o);
+        return bytes;
+    }
+    constexpr int NB = BITS * 8;
+    const int cells = min(n, budget / (16 * NB) + 1), row = lane & 15;
+    const uint8_t* from = p.w + ((rb * 16 + row) * n_cells + c) * NB;
+    const uint8_t* to = from + cells * NB;
+    // whole lines, the first one from the row's own bytes on
+    for (const uint8_t* a = from + 128 * (lane >> 4); a < to; a += 256) ask(a);
+    if (lane >= 16) ask(to - NB);
+    if (SRC == ROWS_SB) {
+        if (lane < cells) ask(p.s + (rb * n_cells + c + lane) * 128);
+    } else {
+        ask((lane < 16 ? p.s : p.b) + ((rb * 16 + row) * ((size_t)(n_cells * 64) >> gshift) + ((c * 64) >> gshift)) * 2);
+    }
+    return cells * 16 * NB;
 }
 // Two bytes of codes (low and high half) -> the bf16 pair of their values: q = 16 * hi + lo, exact.
 FFAI_DEVINL uint32_t byte_pair(uint32_t w, uint32_t mask, uint32_t expo) {
@@ -181,9 +295,10 @@ FFAI_DEVINL uint32_t byte_pair(uint32_t w, uint32_t mask, uint32_t expo) {
     const __nv_bfloat162 q = __hfma2(hi, k16, lo);
     return *reinterpret_cast<const uint32_t*>(&q);
 }
-// The A fragment of MMA hp of 8-run w.  4 bits: pairs are 128 + q (the offset goes into the bias term).
-template <int BITS, bool G32>
-FFAI_DEVINL void a_fragment(const Raw<BITS, G32>& r, int w, int hp, uint32_t mask, uint32_t expo, uint32_t* a) {
+// The A fragment of MMA hp of 8-run w: the pairs (0, 4), (1, 5) or (2, 6), (3, 7) of its k, the order the activations have.
+// 4 bits: pairs are 128 + q (the offset goes into the bias term).
+template <int BITS, bool G32, Source SRC>
+FFAI_DEVINL void a_fragment(const Raw<BITS, G32, SRC>& r, int w, int hp, uint32_t mask, uint32_t expo, uint32_t* a) {
     if (BITS == 4) {
         const uint32_t lo = w ? r.w[0].y : r.w[0].x, hi = w ? r.w[0].w : r.w[0].z;   // rows g, g+8
         a[0] = dmma::and_or(lo >> (8 * hp), mask, expo);
@@ -192,7 +307,8 @@ FFAI_DEVINL void a_fragment(const Raw<BITS, G32>& r, int w, int hp, uint32_t mas
         a[3] = dmma::and_or(hi >> (8 * hp + 4), mask, expo);
     } else {
         const uint4 &x = r.w[0], &y = r.w[BITS == 4 ? 0 : 1];
-        const uint32_t lo = w ? (hp ? x.w : x.z) : (hp ? x.y : x.x), hi = w ? (hp ? y.w : y.z) : (hp ? y.y : y.x);
+        const uint32_t sel = hp ? 0x7632 : 0x5410;   // bytes k0 k1 k4 k5 | k2 k3 k6 k7
+        const uint32_t lo = w ? __byte_perm(x.z, x.w, sel) : __byte_perm(x.x, x.y, sel), hi = w ? __byte_perm(y.z, y.w, sel) : __byte_perm(y.x, y.y, sel);
         a[0] = byte_pair(lo, mask, expo);
         a[1] = byte_pair(hi, mask, expo);
         a[2] = byte_pair(lo >> 8, mask, expo);
@@ -242,8 +358,8 @@ FFAI_DEVINL void column_sums(const uint4* x0, const uint4* x1, float (*sx)[2]) {
 // Adds the cell's contribution to rows g, g+8 (tot[0..1], tot[2..3]) and columns 2t, 2t+1, times the columns' weights
 // with WEIGHTED.  x0, x1: the TERMS terms of the activations; sx[half][column]: run sums.  WEIGHTED leaves a column whose token
 // does not have this expert (`on`) alone: its products are zero, but zero times an infinite scale is not.
-template <int BITS, bool G32, bool WEIGHTED, int TERMS>
-FFAI_DEVINL void cell_dot(const Raw<BITS, G32>& r, uint32_t mask, uint32_t expo, const uint4* x0, const uint4* x1, const float (*sx)[2], float w0,
+template <int BITS, bool G32, Source SRC, bool WEIGHTED, int TERMS>
+FFAI_DEVINL void cell_dot(const Raw<BITS, G32, SRC>& r, uint32_t mask, uint32_t expo, const uint4* x0, const uint4* x1, const float (*sx)[2], float w0,
                           float w1, bool on0, bool on1, float* tot) {
     float c[2][4];
 #pragma unroll
@@ -251,7 +367,7 @@ FFAI_DEVINL void cell_dot(const Raw<BITS, G32>& r, uint32_t mask, uint32_t expo,
 #pragma unroll
         for (int hp = 0; hp < 2; ++hp) {
             uint32_t a[4];
-            a_fragment<BITS, G32>(r, w, hp, mask, expo, a);
+            a_fragment<BITS, G32, SRC>(r, w, hp, mask, expo, a);
 #pragma unroll
             for (int i = TERMS - 1; i >= 0; --i) {
                 const uint4& x = w ? x1[i] : x0[i];
@@ -264,7 +380,7 @@ FFAI_DEVINL void cell_dot(const Raw<BITS, G32>& r, uint32_t mask, uint32_t expo,
     for (int h = 0; h < (G32 ? 2 : 1); ++h)
 #pragma unroll
         for (int i = 0; i < 2; ++i) {   // row half
-            const float sc = __uint_as_float(r.s(h, i) << 16), b = __uint_as_float(r.s(h, i) & 0xFFFF0000u);
+            const float sc = r.scale(h, i), b = r.bias(h, i);
             const float bm = BITS == 4 ? fmaf(-128.0f, sc, b) : b;
 #pragma unroll
             for (int col = 0; col < 2; ++col) {
@@ -307,14 +423,15 @@ struct GridBarrier {
 
 // Where one expert set's gate/up products come from and go to.
 struct GateUp {
-    const uint8_t* stream;
+    Proj gate, up;         // STREAM: gate alone
+    int gshift;
     int I;                 // output rows of each projection
     int u0, n_experts;     // table slots
     const uint16_t *rb_gate, *rb_up;
     int activation;
     float limit, alpha;
     uint16_t* inner;       // rows of I
-    size_t plane;          // elements between the terms of a result
+    uint32_t plane;        // elements between the terms of a result
 };
 
 // n cells cut into WARPS contiguous ranges: the first cell of a warp's range, and the warp whose range holds a cell.
@@ -327,16 +444,15 @@ FFAI_DEVINL int range_owner(int n, int cell) { return (int)((uint32_t)((cell + 1
 // warp + j (ranges are contiguous, so the slots are distinct and an item's are consecutive); after ONE __syncthreads per
 // batch the items are finished by all threads.  (With a __syncthreads per item and every warp on the same item an item
 // took 1.2 us at one token and 2.9 at eight, mostly waiting for the finishing warps.)
-template <int BITS, bool G32, int TERMS>
+template <int BITS, bool G32, Source SRC, int TERMS>
 FFAI_DEVINL void gate_up_phase(const GateUp& a, int T, int H, const Tables* tb, uint32_t x_u, int x_pitch, float* red,
                                int warp, int lane, uint32_t mask, uint32_t expo) {
-    using C = Cell<BITS, G32>;
-    constexpr int AHEAD = C::PAIRS_AHEAD;
+    constexpr int AHEAD = PAIRS_AHEAD;
     const int n_cells = H / 64, n_rb = a.I / 16, n_items = a.n_experts * n_rb;
     const int g = lane >> 2, t = lane & 3;
     const int i_begin = (int)((uint32_t)n_items * blockIdx.x / gridDim.x), i_end = (int)((uint32_t)n_items * (blockIdx.x + 1) / gridDim.x);
     const int tile = 2 * T * RED_PITCH;                                   // floats per slot
-    const int batch = RED_BYTES / 4 / tile - (WARPS - 1);                 // items per batch
+    const int batch = gate_up_batch(T);
 
     for (int i0 = i_begin; i0 < i_end; i0 += batch) {
         const int n_here = min(batch, i_end - i0), flat = n_here * n_cells;
@@ -348,22 +464,21 @@ FFAI_DEVINL void gate_up_phase(const GateUp& a, int T, int H, const Tables* tb, 
             asm volatile("prefetch.global.L2 [%0];" ::"l"(a.rb_gate + rr));
             asm volatile("prefetch.global.L2 [%0];" ::"l"(a.rb_up + rr));
         }
-        // loads run AHEAD pairs in front of the arithmetic; a segment is the rest of the range within one expert's stream
-        struct Pair { Raw<BITS, G32> gate, up; } buf[AHEAD] = {};
-        const uint8_t *src_w = nullptr, *src_s = nullptr;
+        // loads run AHEAD pairs in front of the arithmetic; a segment is the rest of the range within one item (one expert's stream)
+        struct Pair { Raw<BITS, G32, SRC> gate, up; } buf[AHEAD] = {};
+        Cursor<BITS, G32, SRC> cur{};
         int p_q = q0, p_left = 0;
         auto fetch = [&](Pair& d) {
             const bool on = p_q < q1;
             if (p_left == 0 && on) {
                 const int j = p_q / n_cells, it = i0 + j, u = it / n_rb, rb = it - u * n_rb, c = p_q - j * n_cells;
-                const uint8_t* src = a.stream + (((size_t)tb->expert[a.u0 + u] * n_rb + rb) * n_cells + c) * (2 * C::BYTES);
-                src_w = src + lane * 16;
-                src_s = src + C::W + g * (G32 ? 16 : 8);
-                p_left = ((u + 1) * n_rb - i0) * n_cells - p_q;
+                cur.seek(a.gate, tb->expert[a.u0 + u] * (uint32_t)n_rb + rb, n_cells, c, 2, a.gshift, lane);
+                p_left = SRC == STREAM ? ((u + 1) * n_rb - i0) * n_cells - p_q : n_cells - c;
             }
-            load_raw<BITS, G32>(on, src_w, src_s, d.gate);
-            load_raw<BITS, G32>(on, src_w + C::BYTES, src_s + C::BYTES, d.up);
-            src_w += 2 * C::BYTES; src_s += 2 * C::BYTES; --p_left; ++p_q;
+            cur.load(on, a.gate, 0, n_cells, a.gshift, d.gate);
+            cur.load(on, a.up, 1, n_cells, a.gshift, d.up);
+            cur.next(2);
+            --p_left; ++p_q;
         };
 #pragma unroll
         for (int d = 0; d < AHEAD; ++d) fetch(buf[d]);
@@ -395,8 +510,8 @@ FFAI_DEVINL void gate_up_phase(const GateUp& a, int T, int H, const Tables* tb, 
             } else {
                 sx[0][0] = ld_s4(x0); sx[0][1] = ld_s4(x1);
             }
-            cell_dot<BITS, G32, false, 1>(b.gate, mask, expo, &xa, &xb, sx, 0.0f, 0.0f, true, true, tot[0]);
-            cell_dot<BITS, G32, false, 1>(b.up, mask, expo, &xa, &xb, sx, 0.0f, 0.0f, true, true, tot[1]);
+            cell_dot<BITS, G32, SRC, false, 1>(b.gate, mask, expo, &xa, &xb, sx, 0.0f, 0.0f, true, true, tot[0]);
+            cell_dot<BITS, G32, SRC, false, 1>(b.up, mask, expo, &xa, &xb, sx, 0.0f, 0.0f, true, true, tot[1]);
             fetch(b);
             xl += RUN; x0 += RUN; x1 += RUN;
             if (--here == 0) {
@@ -451,13 +566,25 @@ FFAI_DEVINL void gate_up_phase(const GateUp& a, int T, int H, const Tables* tb, 
     }
 }
 
+// The eight values from k on (a multiple of 8) of a quantized row of K: fma(q, scale, bias), any code width.  Eight codes are
+// `bits` whole bytes of the LSB-first stream.
+FFAI_DEVINL void affine_run8(const uint32_t* w, const uint16_t* scales, const uint16_t* biases, int bits, int group, int k, int K, float* v) {
+    const int byte = k / 8 * bits, i = byte >> 2, shift = (byte & 3) * 8, last = K * bits / 32 - 1;
+    const uint32_t a = w[i], b = w[min(i + 1, last)], c = w[min(i + 2, last)];   // (codes of words past the end are not used)
+    const uint64_t codes = (uint64_t)__funnelshift_r(a, b, shift) | ((uint64_t)__funnelshift_r(b, c, shift) << 32);
+    const float s = bf16_bits_to_f32(scales[k / group]), o = bf16_bits_to_f32(biases[k / group]);
+    const uint32_t mask = (1u << bits) - 1;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = fmaf((float)((uint32_t)(codes >> (j * bits)) & mask), s, o);
+}
+
 // SBITS: bit width of the shared expert (4 or 8, group 64 or 128), 0 without one.
 template <int BITS, bool G32, int SBITS>
 __global__ void __launch_bounds__(THREADS, 1)
 fused_decode_kernel(const Params p) {
     using L = Layout<BITS, G32>;
-    using C = Cell<BITS, G32>;
-    using CS = Cell<SBITS == 0 ? 4 : SBITS, false>;
+    constexpr Source SRC = SOURCE<BITS, G32>;
+    constexpr int SB = SBITS == 0 ? 4 : SBITS;
     extern __shared__ __align__(128) uint8_t smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
@@ -566,20 +693,31 @@ fused_decode_kernel(const Params p) {
     }
     if (SBITS != 0 && p.sh_gate_kind != 0 && blockIdx.x == gridDim.x - 1 && warp < T) {
         float acc = 0.0f;
-        for (int k = lane * 8; k < H; k += 256) {
+        auto run = [&](int k, const float* wf) {
             const uint4 xv = *reinterpret_cast<const uint4*>(p.x + (size_t)warp * H + k);
             const float xf[8] = {bf16lo(xv.x), bf16hi(xv.x), bf16lo(xv.y), bf16hi(xv.y), bf16lo(xv.z), bf16hi(xv.z), bf16lo(xv.w), bf16hi(xv.w)};
-            float wf[8];
-            if (p.sh_gate_kind == 1) {
-                const float4 w0 = *reinterpret_cast<const float4*>((const float*)p.sh_gate_w + k), w1 = *reinterpret_cast<const float4*>((const float*)p.sh_gate_w + k + 4);
-                wf[0] = w0.x; wf[1] = w0.y; wf[2] = w0.z; wf[3] = w0.w; wf[4] = w1.x; wf[5] = w1.y; wf[6] = w1.z; wf[7] = w1.w;
-            } else {
-                const uint4 w = *reinterpret_cast<const uint4*>((const uint16_t*)p.sh_gate_w + k);
-                wf[0] = bf16lo(w.x); wf[1] = bf16hi(w.x); wf[2] = bf16lo(w.y); wf[3] = bf16hi(w.y);
-                wf[4] = bf16lo(w.z); wf[5] = bf16hi(w.z); wf[6] = bf16lo(w.w); wf[7] = bf16hi(w.w);
-            }
 #pragma unroll
             for (int j = 0; j < 8; ++j) acc = fmaf(wf[j], xf[j], acc);
+        };
+        if (p.sh_gate_kind == 3) {
+#pragma unroll 4
+            for (int k = lane * 8; k < H; k += 256) {
+                float wf[8];
+                affine_run8((const uint32_t*)p.sh_gate_w, p.sh_gate_s, p.sh_gate_b, p.sh_gate_bits, p.sh_gate_group, k, H, wf);
+                run(k, wf);
+            }
+        } else if (p.sh_gate_kind == 1) {
+            for (int k = lane * 8; k < H; k += 256) {
+                const float4 w0 = *reinterpret_cast<const float4*>((const float*)p.sh_gate_w + k), w1 = *reinterpret_cast<const float4*>((const float*)p.sh_gate_w + k + 4);
+                const float wf[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+                run(k, wf);
+            }
+        } else {
+            for (int k = lane * 8; k < H; k += 256) {
+                const uint4 w = *reinterpret_cast<const uint4*>((const uint16_t*)p.sh_gate_w + k);
+                const float wf[8] = {bf16lo(w.x), bf16hi(w.x), bf16lo(w.y), bf16hi(w.y), bf16lo(w.z), bf16hi(w.z), bf16lo(w.w), bf16hi(w.w)};
+                run(k, wf);
+            }
         }
         acc = warp_sum(acc);
         if (lane == 0) p.sh_gate_logit[warp] = acc;
@@ -593,8 +731,8 @@ fused_decode_kernel(const Params p) {
             if (threadIdx.x == 0) { tb->expert[SHARED_U] = 0; tb->base[SHARED_U] = 0; tb->cnt[SHARED_U] = (uint16_t)T; }
         }
         __syncthreads();
-        const GateUp a{p.sh_gate_up, p.Is, SHARED_U, 1, nullptr, nullptr, 0, 0.0f, 0.0f, p.sh_inner, p.sh_plane};
-        gate_up_phase<SBITS == 0 ? 4 : SBITS, false, SH_TERMS>(a, T, H, tb, x_u, x_pitch, red, warp, lane, mask, expo);
+        const GateUp a{p.sh_gate, p.sh_up, p.sh_gshift, p.Is, SHARED_U, 1, nullptr, nullptr, 0, 0.0f, 0.0f, p.sh_inner, p.sh_plane};
+        gate_up_phase<SB, false, ROWS, SH_TERMS>(a, T, H, tb, x_u, x_pitch, red, warp, lane, mask, expo);
     }
     if (!bar.wait(&tb->failed)) {
         if (threadIdx.x == 0) atomicExch(p.error_word, (uint32_t)ERR_GRID_BARRIER);
@@ -652,8 +790,8 @@ fused_decode_kernel(const Params p) {
 
     // ── phase 3: gate/up of the routed experts ──
     {
-        const GateUp a{p.gate_up, I, 0, U, p.rb_gate, p.rb_up, p.activation, p.limit, p.alpha, p.inner, p.inner_plane};
-        gate_up_phase<BITS, G32, INNER_TERMS<BITS>>(a, T, H, tb, x_u, x_pitch, red, warp, lane, mask, expo);
+        const GateUp a{p.gate, p.up, p.gshift, I, 0, U, p.rb_gate, p.rb_up, p.activation, p.limit, p.alpha, p.inner, p.inner_plane};
+        gate_up_phase<BITS, G32, SRC, INNER_TERMS<BITS>>(a, T, H, tb, x_u, x_pitch, red, warp, lane, mask, expo);
     }
 
     // ── phase 4: down over all experts of a 16-row block ──
@@ -689,19 +827,14 @@ fused_decode_kernel(const Params p) {
             if (++w.u > U || cells_of(w.u) == 0) { w.u = 0; ++w.item; }
         }
     };
-    auto weights_at = [&](const Walk& w) {
-        return w.u == U ? p.sh_down + ((size_t)w.item * cs + w.c) * CS::BYTES
-                        : p.down + (((size_t)tb->expert[w.u] * n_rb + w.item) * ci + w.c) * C::BYTES;
-    };
     // the first 8 KB of the warp's weights (all of them at one token) on their way into L2 across the barrier
     {
         Walk w = walk_to(q0);
         int budget = 8192;
         for (int q = q0; q < q1 && budget > 0;) {
-            const int n = min(cells_of(w.u) - w.c, q1 - q), bytes = min(n * (w.u == U ? CS::BYTES : C::BYTES), budget);
-            const uint8_t* src = weights_at(w);
-            for (int o = lane * 128; o < bytes; o += 32 * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(src + o));
-            budget -= bytes;
+            const int n = min(cells_of(w.u) - w.c, q1 - q);
+            if (SBITS != 0 && w.u == U) budget -= prefetch_cells<SB, false, ROWS>(p.sh_down, w.item, cs, w.c, n, p.sh_gshift, budget, lane);
+            else budget -= prefetch_cells<BITS, G32, SRC>(p.down, (size_t)tb->expert[w.u] * n_rb + w.item, ci, w.c, n, p.gshift, budget, lane);
             q += n;
             advance(w, n);
         }
@@ -720,30 +853,33 @@ fused_decode_kernel(const Params p) {
     // the cells [c, c + n) of one expert: weights and activation fragments are loaded CELLS_AHEAD cells in front
     auto run_cells = [&](auto shared_tag, const Walk& w, int n) {
         constexpr bool SH = decltype(shared_tag)::value;
-        using CC = std::conditional_t<SH, CS, C>;
-        constexpr int B = SH ? (SBITS == 0 ? 4 : SBITS) : BITS;
+        constexpr int B = SH ? SB : BITS;
         constexpr bool H32 = SH ? false : G32;
         constexpr int TERMS = SH ? SH_TERMS : INNER_TERMS<BITS>;
-        constexpr int AHEAD = TERMS == 3 ? 2 : CC::CELLS_AHEAD;
-        const size_t plane = SH ? p.sh_plane : p.inner_plane;
+        constexpr Source S = SH ? ROWS : SRC;
+        constexpr int AHEAD = TERMS == 3 ? 2 : CELLS_AHEAD;
+        const uint32_t plane = SH ? p.sh_plane : p.inner_plane;
         const int u = SH ? SHARED_U : w.u;
         const int row = tb->pos[u][g], ld = SH ? p.Is : I;
         const float w0 = tb->colw[u][2 * t], w1 = tb->colw[u][2 * t + 1];
         const bool on0 = tb->pos[u][2 * t] >= 0, on1 = tb->pos[u][2 * t + 1] >= 0;
         // columns without this expert: zero fragments
         const uint16_t* xp = (SH ? p.sh_inner : p.inner) + (size_t)max(row, 0) * ld + w.c * 64 + (H32 ? 8 : 16) * t;
-        const uint8_t *src_w = weights_at(w) + lane * 16, *src_s = weights_at(w) + CC::W + g * (H32 ? 16 : 8);
-        struct Ahead { Raw<B, H32> raw; uint4 x0[TERMS], x1[TERMS]; } buf[AHEAD] = {};   // (columns without a row keep zeros)
+        const Proj& proj = SH ? p.sh_down : p.down;
+        const int cells = SH ? cs : ci, gshift = SH ? p.sh_gshift : p.gshift;
+        Cursor<B, H32, S> cur;
+        cur.seek(proj, SH ? (uint32_t)w.item : tb->expert[w.u] * (uint32_t)n_rb + w.item, cells, w.c, 1, gshift, lane);
+        struct Ahead { Raw<B, H32, S> raw; uint4 x0[TERMS], x1[TERMS]; } buf[AHEAD] = {};   // (columns without a row keep zeros)
         int p_n = n;
         auto fetch = [&](Ahead& d) {
             const bool on = p_n > 0;
-            load_raw<B, H32>(on, src_w, src_s, d.raw);
+            cur.load(on, proj, 0, cells, gshift, d.raw);
 #pragma unroll
             for (int i = 0; i < TERMS; ++i) {
                 ldcg16_if(on && row >= 0, xp + i * plane, d.x0[i]);
                 ldcg16_if(on && row >= 0, xp + i * plane + (H32 ? 32 : 8), d.x1[i]);
             }
-            src_w += CC::BYTES; src_s += CC::BYTES; xp += 64; --p_n;
+            cur.next(1); xp += 64; --p_n;
         };
 #pragma unroll
         for (int d = 0; d < AHEAD; ++d) fetch(buf[d]);
@@ -753,7 +889,7 @@ fused_decode_kernel(const Params p) {
             for (int d = 0; d < AHEAD; ++d) {
                 float sx[2][2];
                 column_sums<H32, TERMS>(buf[d].x0, buf[d].x1, sx);
-                cell_dot<B, H32, true, TERMS>(buf[d].raw, mask, expo, buf[d].x0, buf[d].x1, sx, w0, w1, on0, on1, tot);
+                cell_dot<B, H32, S, true, TERMS>(buf[d].raw, mask, expo, buf[d].x0, buf[d].x1, sx, w0, w1, on0, on1, tot);
                 fetch(buf[d]);
                 if (--n == 0) break;
             }
@@ -829,51 +965,6 @@ fused_decode_kernel(const Params p) {
             p.plan.offsets[e] = less;
             if (e < E) p.plan.counts[e] = same;
         }
-}
-
-// Load-time re-tiling of one stacked projection (pair) into cells, for the formats that expert_stream_decode.cuh does
-// not lay out (8-bit codes, groups of 32).  One block per cell, thread = one row of the cell (two threads halves).
-//   out[((e*n_rb + rb)*n_cells + cell) * NP * BYTES + proj * BYTES],  NP = 2 with a second projection
-template <int BITS, bool G32>
-__global__ void retile_cell_kernel(const uint32_t* __restrict__ w1, const uint16_t* __restrict__ s1, const uint16_t* __restrict__ b1,
-                                   const uint32_t* __restrict__ w2, const uint16_t* __restrict__ s2, const uint16_t* __restrict__ b2,
-                                   uint8_t* __restrict__ out, int N, int K, int group_size) {
-    using C = Cell<BITS, G32>;
-    const int np = w2 ? 2 : 1;
-    const int n_cells = K / 64, wpr = K * BITS / 32, gpr = K / group_size;
-    const size_t cell_id = blockIdx.x;
-    const int cell = (int)(cell_id % n_cells);
-    const size_t row0 = (cell_id / n_cells) * 16;
-    for (int q = 0; q < np; ++q) {
-        const uint32_t* w = q ? w2 : w1;
-        const uint16_t* s = q ? s2 : s1;
-        const uint16_t* b = q ? b2 : b1;
-        uint8_t* dst = out + (cell_id * np + q) * C::BYTES;
-        const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-        if (threadIdx.x < 64) {
-            const int h = threadIdx.x >> 5;                   // row half
-            const uint32_t* src = w + (row0 + g + 8 * h) * wpr + cell * (2 * BITS);
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                const int run = G32 ? t + 4 * i : 2 * t + i;  // the lane's 8-runs
-                if (BITS == 4) {
-                    reinterpret_cast<uint32_t*>(dst)[lane * 4 + 2 * h + i] = src[run];
-                } else {
-                    const uint32_t lo = src[2 * run], hi = src[2 * run + 1];   // k0..k3, k4..k7
-                    uint32_t* d = reinterpret_cast<uint32_t*>(dst + h * 512) + lane * 4 + 2 * i;
-                    d[0] = __byte_perm(lo, hi, 0x5410);       // k0 k1 k4 k5
-                    d[1] = __byte_perm(lo, hi, 0x7632);       // k2 k3 k6 k7
-                }
-            }
-        } else if (threadIdx.x < 64 + 16) {
-            const int r = threadIdx.x - 64, gg = r & 7, h = r >> 3;
-            uint32_t* d = reinterpret_cast<uint32_t*>(dst + C::W);
-            for (int f = 0; f < (G32 ? 2 : 1); ++f) {
-                const size_t at = (row0 + r) * gpr + (cell * 64 + 32 * f) / group_size;
-                d[gg * (G32 ? 4 : 2) + 2 * f + h] = (uint32_t)s[at] | ((uint32_t)b[at] << 16);
-            }
-        }
-    }
 }
 
 }  // namespace fdec

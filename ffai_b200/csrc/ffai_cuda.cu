@@ -82,11 +82,6 @@ struct ffai_moe_layer {
     uint8_t* st_down = nullptr;      // ... and down (re-tiled copies of the packed experts, owned with the weights)
     // one-launch forward of the smallest batches (expert_fused_decode.cuh)
     bool fused_planned = false;
-    const uint8_t* fd_gate_up = nullptr;     // cells of the routed experts (4-bit group 64/128: the streams above) ...
-    const uint8_t* fd_down = nullptr;
-    const uint8_t* fd_sh_gate_up = nullptr;  // ... and of the shared expert
-    const uint8_t* fd_sh_down = nullptr;
-    const float* fd_sh_gate_f32 = nullptr;   // a quantized shared-expert gate expanded to fp32
     uint16_t* fd_inner = nullptr;            // [terms][fdec::MAX_ROWS, I] activation results
     uint16_t* fd_sh_inner = nullptr;         // [terms][fdec::MAX_T, Is]
     float* fd_split = nullptr;               // [2 * SMs][16 * fdec::MAX_T]
@@ -575,20 +570,6 @@ bool launch_fused_decode(const fdec::Params& p, int bits, bool g32, int shared_b
     return g32 ? launch_fused_decode_s<8, true>(p, shared_bits, n_sms, st) : launch_fused_decode_s<8, false>(p, shared_bits, n_sms, st);
 }
 
-// One projection (w2 == nullptr) or a gate/up pair re-tiled into the cells of the one-launch decode kernel.
-int launch_retile_cells(const ffai_qproj& a, const ffai_qproj* b, uint8_t* out, size_t n_groups, int N, int K, int bits, int gs) {
-    const unsigned cells = (unsigned)(n_groups * (N / 16) * (K / 64));
-    const uint32_t* w2 = b ? b->weight : nullptr;
-    const uint16_t* s2 = b ? b->scales : nullptr;
-    const uint16_t* b2 = b ? b->biases : nullptr;
-    if (bits == 4 && gs == 32) fdec::retile_cell_kernel<4, true><<<cells, 96>>>(a.weight, a.scales, a.biases, w2, s2, b2, out, N, K, gs);
-    else if (bits == 4) fdec::retile_cell_kernel<4, false><<<cells, 96>>>(a.weight, a.scales, a.biases, w2, s2, b2, out, N, K, gs);
-    else if (gs == 32) fdec::retile_cell_kernel<8, true><<<cells, 96>>>(a.weight, a.scales, a.biases, w2, s2, b2, out, N, K, gs);
-    else fdec::retile_cell_kernel<8, false><<<cells, 96>>>(a.weight, a.scales, a.biases, w2, s2, b2, out, N, K, gs);
-    return cudaGetLastError() == cudaSuccess ? FFAI_OK : FFAI_ERR_CUDA;
-}
-size_t cell_bytes(int bits, int gs) { return (bits == 4 ? 512 : 1024) + (gs == 32 ? 128 : 64); }
-
 // dense [1,H] projection per token (shared-expert gate stored as f32 / bf16)
 template <typename TW>
 __global__ void dense_rowdot_kernel(const TW* __restrict__ w, const uint16_t* __restrict__ x,
@@ -913,13 +894,15 @@ extern "C" FFAI_API int ffai_moe_create(const ffai_moe_config* config, ffai_moe_
     if (world > 1 && !L->xg && (rc = ws_alloc(L, &L->xg, Mx * H))) return rc;  // regrouped rows for the GEMV path
     L->fused_planned = world == 1 && cc_major == 10 && !L->no_gate && (c.expert_bits == 4 || c.expert_bits == 8) &&
                        (c.shared_intermediate == 0 || ((c.shared_bits == 4 || c.shared_bits == 8) && c.shared_group_size != 32));
-    if (L->fused_planned) {
+    if (L->fused_planned) {   // without room for its buffers the layer keeps to the launch chain
         const int terms = c.expert_bits == 8 ? fdec::INNER_TERMS<8> : fdec::INNER_TERMS<4>;
-        if ((rc = ws_alloc(L, &L->fd_inner, terms * fdec::MAX_ROWS * I))) return rc;
-        if ((rc = ws_alloc(L, &L->fd_sh_inner, (size_t)fdec::SH_TERMS * fdec::MAX_T * c.shared_intermediate))) return rc;
-        if ((rc = ws_alloc(L, &L->fd_split, (size_t)2 * L->n_sms * 16 * fdec::MAX_T))) return rc;
-        if ((rc = ws_alloc(L, &L->fd_sync, 1 + H / 16))) return rc;
-        CUDA_TRY(L, cudaMemset(L->fd_sync, 0, (1 + H / 16) * 4));
+        if (ws_alloc(L, &L->fd_inner, terms * fdec::MAX_ROWS * I) || ws_alloc(L, &L->fd_sh_inner, (size_t)fdec::SH_TERMS * fdec::MAX_T * c.shared_intermediate) ||
+            ws_alloc(L, &L->fd_split, (size_t)2 * L->n_sms * 16 * fdec::MAX_T) || ws_alloc(L, &L->fd_sync, 1 + H / 16)) {
+            L->fused_planned = false;
+            cudaGetLastError();
+        } else {
+            CUDA_TRY(L, cudaMemset(L->fd_sync, 0, (1 + H / 16) * 4));
+        }
     }
     return FFAI_OK;
 }
@@ -1086,47 +1069,6 @@ extern "C" FFAI_API int ffai_moe_set_weights(ffai_moe_layer* L, const ffai_moe_w
             L->st_gate_up = static_cast<uint8_t*>(a);
             L->st_down = static_cast<uint8_t*>(b);
         }
-    }
-    // cells of the one-launch decode kernel (formats the streams above do not cover, and the shared expert)
-    L->fd_gate_up = L->fd_down = L->fd_sh_gate_up = L->fd_sh_down = nullptr;
-    L->fd_sh_gate_f32 = nullptr;
-    if (L->fused_planned) {
-        auto cells = [&](const ffai_qproj& a, const ffai_qproj* b, size_t n, int N, int K, int bits, int gs, const uint8_t** out) -> int {
-            const size_t count = n * (N / 16) * (K / 64);
-            if (count >= (1u << 31)) return FFAI_OK;   // the layer then keeps to the launch chain
-            void* buf = nullptr;
-            if (cudaMalloc(&buf, count * (b ? 2 : 1) * cell_bytes(bits, gs)) != cudaSuccess) {   // no room for a copy: the launch chain
-                cudaGetLastError();
-                return FFAI_OK;
-            }
-            L->owned_weights.push_back(buf);
-            if (launch_retile_cells(a, b, static_cast<uint8_t*>(buf), n, N, K, bits, gs)) return fail(L, FFAI_ERR_CUDA, "re-tiling the experts failed");
-            *out = static_cast<const uint8_t*>(buf);
-            return FFAI_OK;
-        };
-        const int H = c.hidden, I = c.intermediate, Is = c.shared_intermediate;
-        if (L->st_gate_up) {
-            L->fd_gate_up = L->st_gate_up;
-            L->fd_down = L->st_down;
-        } else {
-            if ((rc = cells(L->w.gate_proj, &L->w.up_proj, El, I, H, c.expert_bits, c.expert_group_size, &L->fd_gate_up))) return rc;
-            if ((rc = cells(L->w.down_proj, nullptr, El, H, I, c.expert_bits, c.expert_group_size, &L->fd_down))) return rc;
-        }
-        if (Is > 0) {
-            if ((rc = cells(L->w.shared_gate_proj, &L->w.shared_up_proj, 1, Is, H, c.shared_bits, c.shared_group_size, &L->fd_sh_gate_up))) return rc;
-            if ((rc = cells(L->w.shared_down_proj, nullptr, 1, H, Is, c.shared_bits, c.shared_group_size, &L->fd_sh_down))) return rc;
-            if (c.shared_gate_kind == FFAI_LINEAR_AFFINE) {
-                void* buf = nullptr;
-                CUDA_TRY(L, cudaMalloc(&buf, (size_t)H * sizeof(float)));
-                L->owned_weights.push_back(buf);
-                const uint32_t* gw = static_cast<const uint32_t*>(L->w.shared_gate.weight);
-                BITS_SWITCH(c.shared_gate_bits, (expand_router_f32_kernel<B><<<(H + 255) / 256, 256>>>(gw, L->w.shared_gate.scales, L->w.shared_gate.biases,
-                                                                                                     static_cast<float*>(buf), 1, H, c.shared_gate_group_size)));
-                L->fd_sh_gate_f32 = static_cast<const float*>(buf);
-            }
-        }
-        CUDA_TRY(L, cudaGetLastError());
-        CUDA_TRY(L, cudaDeviceSynchronize());
     }
     L->weights_set = true;
     return FFAI_OK;
@@ -1731,25 +1673,38 @@ int forward_device(ffai_moe_layer* L, const uint16_t* x, int T, uint16_t* out, c
 
     // The smallest batches: the whole block in one launch.  Stage events need launches to sit between, and the options
     // that pick or tune one of the other decode kernels mean those kernels.
-    if (T <= fdec::MAX_T && M <= fdec::MAX_ROWS && L->fd_gate_up && L->fd_down && (c.shared_intermediate == 0 || (L->fd_sh_gate_up && L->fd_sh_down)) &&
+    if (T <= fdec::MAX_T && M <= fdec::MAX_ROWS && L->fused_planned && (L->st_gate_up || c.expert_bits == 8 || c.expert_group_size == 32) &&
         (L->opt_path == 0 || L->opt_path == 3) && L->opt_decode == 0 && L->opt_ksplit == 0 && L->opt_decode_team == 0 && !L->timing) {
         fdec::Params p{};
         p.rp = router_params(L);
         p.x = x; p.xr = L->router_x ? L->router_x : x;
         p.T = T; p.H = H; p.I = I;
-        p.gate_up = L->fd_gate_up; p.down = L->fd_down;
+        auto bytes = [](const void* q) { return static_cast<const uint8_t*>(q); };
+        auto rows = [&](const ffai_qproj& q) { return fdec::Proj{bytes(q.weight), bytes(q.scales), bytes(q.biases)}; };
+        auto log2_of = [](int group) { return group == 32 ? 5 : (group == 64 ? 6 : 7); };
+        p.gshift = log2_of(c.expert_group_size);
+        p.gate = rows(L->w.gate_proj); p.up = rows(L->w.up_proj); p.down = rows(L->w.down_proj);
+        if (c.expert_bits == 4 && c.expert_group_size == 32) {
+            p.gate.s = bytes(L->sb_gate); p.up.s = bytes(L->sb_up); p.down.s = bytes(L->sb_down);
+        } else if (c.expert_bits == 4) {
+            p.gate = p.up = fdec::Proj{L->st_gate_up, nullptr, nullptr};
+            p.down = fdec::Proj{L->st_down, nullptr, nullptr};
+        }
         p.rb_gate = L->w.gate_proj.row_bias; p.rb_up = L->w.up_proj.row_bias; p.rb_down = L->w.down_proj.row_bias;
         p.activation = c.activation; p.limit = c.swiglu_limit; p.alpha = c.swiglu_alpha;
-        p.Is = c.shared_intermediate; p.sh_gate_up = L->fd_sh_gate_up; p.sh_down = L->fd_sh_down;
+        p.Is = c.shared_intermediate;
         if (p.Is > 0) {
-            p.sh_gate_kind = c.shared_gate_kind == FFAI_LINEAR_NONE ? 0 : (c.shared_gate_kind == FFAI_LINEAR_BF16 ? 2 : 1);
-            p.sh_gate_w = L->fd_sh_gate_f32 ? L->fd_sh_gate_f32 : L->w.shared_gate.weight;
+            p.sh_gate = rows(L->w.shared_gate_proj); p.sh_up = rows(L->w.shared_up_proj); p.sh_down = rows(L->w.shared_down_proj);
+            p.sh_gshift = log2_of(c.shared_group_size);
+            p.sh_gate_kind = c.shared_gate_kind;
+            p.sh_gate_w = L->w.shared_gate.weight; p.sh_gate_s = L->w.shared_gate.scales; p.sh_gate_b = L->w.shared_gate.biases;
+            p.sh_gate_bits = c.shared_gate_bits; p.sh_gate_group = c.shared_gate_group_size;
             p.sh_gate_logit = L->sh_gate;
         }
         p.logits = L->logits; p.indices = L->indices; p.rweights = L->rweights;
         p.plan = PlanOut{L->counts, L->offsets, L->perm, L->inv_perm, nullptr};
         p.inner = L->fd_inner; p.sh_inner = L->fd_sh_inner;
-        p.inner_plane = (size_t)fdec::MAX_ROWS * I; p.sh_plane = (size_t)fdec::MAX_T * c.shared_intermediate;
+        p.inner_plane = fdec::MAX_ROWS * (uint32_t)I; p.sh_plane = fdec::MAX_T * (uint32_t)c.shared_intermediate;
         p.residual = residual; p.out = out;
         p.split = L->fd_split; p.barrier = L->fd_sync; p.tickets = L->fd_sync + 1; p.error_word = L->error_word;
         if (launch_fused_decode(p, c.expert_bits, c.expert_group_size == 32, c.shared_intermediate > 0 ? c.shared_bits : 0, L->n_sms, st)) {

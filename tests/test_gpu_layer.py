@@ -606,3 +606,28 @@ def test_one_launch_confines_non_finite_weights(oracle_mod, bits, gs, field, val
         layer.close()
     assert np.array_equal(dbg.indices, ref.indices)
     assert_parity(out[~has], ref.out_f32[~has], what=spec.name)
+
+
+# 4-bit experts of group 32 add re-tiled scale words (as large as scales and biases) for the decode kernels, 8-bit ones nothing
+@pytest.mark.parametrize("bits,gs,extra", [(8, 64, 0.0), (8, 32, 0.0), (4, 32, 0.2)])
+def test_loading_makes_no_further_copy_of_the_experts(bits, gs, extra):
+    import torch
+    spec = synth.LayerSpec("no_copy", 1024, 768, 24, 4, expert_bits=bits, expert_group_size=gs, shared_intermediate=1024, shared_bits=8,
+                           shared_group_size=64)
+    small = spec.with_(n_experts=4)
+    warm = MoELayer(synth.make_layer(small, 1), 8)      # kernels are loaded on first use
+    warm.forward_host(synth.make_tokens(3, spec.hidden, 1))
+    host = synth.make_layer(spec, 1)
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    layer = MoELayer(host, 8)
+    try:
+        used = before - torch.cuda.mem_get_info()[0]
+        layer.forward_host(synth.make_tokens(3, spec.hidden, 1))
+        assert layer.launch_count() == 1
+    finally:
+        layer.close()
+        warm.close()
+    shared_bf16 = 3 * 1024 * 1024 * 2                   # the shared expert's operand tiles of the prefill path
+    # the rest: workspace of 8 tokens and the 2 MB granules of a few dozen small allocations
+    assert used <= host.weight_bytes() * (1 + extra) + shared_bf16 + (24 << 20), f"{used / 2**20:.0f} MiB for {host.weight_bytes() / 2**20:.0f} MiB of weights"
