@@ -42,7 +42,7 @@ def stale() -> bool:
     if not OUT.exists():
         return True
     t = OUT.stat().st_mtime
-    deps = list(SRC.glob("*.cu")) + list(SRC.glob("*.cuh")) + list(INCLUDE.glob("*.h"))
+    deps = list(SRC.glob("*.cu")) + list(SRC.glob("*.cuh")) + list(SRC.glob("*.hpp")) + list(INCLUDE.glob("*.h"))
     return any(d.stat().st_mtime > t for d in deps)
 
 

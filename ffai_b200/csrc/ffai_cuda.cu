@@ -14,6 +14,7 @@
 
 #include "combine.cuh"
 #include "common.cuh"
+#include "coop_launch.hpp"
 #include "expert_fused_decode.cuh"
 #include "expert_gemv.cuh"
 #include "ep.cuh"
@@ -541,15 +542,15 @@ bool launch_stream_decode(const dstr::Params& p, int team, int n_sms, cudaStream
 }
 
 // The whole block in one cooperative launch (its CTAs meet at grid barriers, so all of them must be resident: one per SM).
-// Returns false when the shape does not fit; the caller then takes the launch chain.
+// Shapes that do not fit, and streams that may not run all of them at once, take the launch chain.
 template <int BITS, bool G32, int SBITS>
-bool launch_fused_decode_t(const fdec::Params& p, int n_sms, cudaStream_t st) {
+CoopLaunch launch_fused_decode_t(const fdec::Params& p, int n_sms, cudaStream_t st, cudaError_t* status) {
     using LY = fdec::Layout<BITS, G32>;
     const int smem = LY::total(p.T, p.H);
-    if (smem > 227 * 1024 || !LY::fits(p.T, p.T * p.rp.top_k, p.rp.n_experts, p.H, p.I, p.Is, p.rp.kind == FFAI_LINEAR_F32 ? 4 : 2, n_sms)) return false;
+    const bool fits = smem <= 227 * 1024 &&
+                      LY::fits(p.T, p.T * p.rp.top_k, p.rp.n_experts, p.H, p.I, p.Is, p.rp.kind == FFAI_LINEAR_F32 ? 4 : 2, n_sms);
     auto k = fdec::fused_decode_kernel<BITS, G32, SBITS>;
     static SmemOptIn opt_in;
-    if (!opt_in.ensure(k, smem)) return false;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(n_sms); cfg.blockDim = dim3(fdec::THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = st;
     cudaLaunchAttribute attr[1];
@@ -557,17 +558,17 @@ bool launch_fused_decode_t(const fdec::Params& p, int n_sms, cudaStream_t st) {
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k, p) == cudaSuccess;
+    return try_cooperative(fits, [&] { return opt_in.ensure(k, smem); }, [&] { return cudaLaunchKernelEx(&cfg, k, p); }, [] { cudaGetLastError(); }, status);
 }
 template <int BITS, bool G32>
-bool launch_fused_decode_s(const fdec::Params& p, int shared_bits, int n_sms, cudaStream_t st) {
-    if (shared_bits == 4) return launch_fused_decode_t<BITS, G32, 4>(p, n_sms, st);
-    if (shared_bits == 8) return launch_fused_decode_t<BITS, G32, 8>(p, n_sms, st);
-    return launch_fused_decode_t<BITS, G32, 0>(p, n_sms, st);
+CoopLaunch launch_fused_decode_s(const fdec::Params& p, int shared_bits, int n_sms, cudaStream_t st, cudaError_t* status) {
+    if (shared_bits == 4) return launch_fused_decode_t<BITS, G32, 4>(p, n_sms, st, status);
+    if (shared_bits == 8) return launch_fused_decode_t<BITS, G32, 8>(p, n_sms, st, status);
+    return launch_fused_decode_t<BITS, G32, 0>(p, n_sms, st, status);
 }
-bool launch_fused_decode(const fdec::Params& p, int bits, bool g32, int shared_bits, int n_sms, cudaStream_t st) {
-    if (bits == 4) return g32 ? launch_fused_decode_s<4, true>(p, shared_bits, n_sms, st) : launch_fused_decode_s<4, false>(p, shared_bits, n_sms, st);
-    return g32 ? launch_fused_decode_s<8, true>(p, shared_bits, n_sms, st) : launch_fused_decode_s<8, false>(p, shared_bits, n_sms, st);
+CoopLaunch launch_fused_decode(const fdec::Params& p, int bits, bool g32, int shared_bits, int n_sms, cudaStream_t st, cudaError_t* status) {
+    if (bits == 4) return g32 ? launch_fused_decode_s<4, true>(p, shared_bits, n_sms, st, status) : launch_fused_decode_s<4, false>(p, shared_bits, n_sms, st, status);
+    return g32 ? launch_fused_decode_s<8, true>(p, shared_bits, n_sms, st, status) : launch_fused_decode_s<8, false>(p, shared_bits, n_sms, st, status);
 }
 
 // dense [1,H] projection per token (shared-expert gate stored as f32 / bf16)
@@ -1707,11 +1708,13 @@ int forward_device(ffai_moe_layer* L, const uint16_t* x, int T, uint16_t* out, c
         p.inner_plane = fdec::MAX_ROWS * (uint32_t)I; p.sh_plane = fdec::MAX_T * (uint32_t)c.shared_intermediate;
         p.residual = residual; p.out = out;
         p.split = L->fd_split; p.barrier = L->fd_sync; p.tickets = L->fd_sync + 1; p.error_word = L->error_word;
-        if (launch_fused_decode(p, c.expert_bits, c.expert_group_size == 32, c.shared_intermediate > 0 ? c.shared_bits : 0, L->n_sms, st)) {
+        cudaError_t status;
+        const CoopLaunch done = launch_fused_decode(p, c.expert_bits, c.expert_group_size == 32, c.shared_intermediate > 0 ? c.shared_bits : 0, L->n_sms, st, &status);
+        if (done == CoopLaunch::failed) return fail(L, FFAI_ERR_CUDA, "one-launch decode failed to launch: %s", cudaGetErrorString(status));
+        if (done == CoopLaunch::ran) {
             L->launches = 1;
             return FFAI_OK;
         }
-        if (cudaGetLastError() != cudaSuccess) return fail(L, FFAI_ERR_CUDA, "one-launch decode failed to launch");
     }
 
     // The shared expert reads only the layer's input.  With a prefill-sized batch (or under expert parallelism) it runs

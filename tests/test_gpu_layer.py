@@ -631,3 +631,43 @@ def test_loading_makes_no_further_copy_of_the_experts(bits, gs, extra):
     shared_bf16 = 3 * 1024 * 1024 * 2                   # the shared expert's operand tiles of the prefill path
     # the rest: workspace of 8 tokens and the 2 MB granules of a few dozen small allocations
     assert used <= host.weight_bytes() * (1 + extra) + shared_bf16 + (24 << 20), f"{used / 2**20:.0f} MiB for {host.weight_bytes() / 2**20:.0f} MiB of weights"
+
+
+def test_stream_with_a_part_of_the_sms_takes_the_launch_chain(oracle_mod):
+    """A green context's stream may run on 64 SMs: one CTA per SM of the device cannot be resident there at once."""
+    import torch
+    cu = pytest.importorskip("cuda.bindings.driver")
+
+    def ok(r):
+        assert int(r[0]) == 0, r[0]
+        return r[1] if len(r) == 2 else r[1:]
+    spec = synth.LayerSpec("part_of_sms", 512, 256, 16, 4)
+    host = synth.make_layer(spec, 41)
+    x = synth.make_tokens(3, spec.hidden, 41)
+    ref = oracle_mod.moe_forward(host, x)
+    layer = MoELayer(host, 8)
+    try:
+        xd = to_dev(x)
+        out = torch.zeros_like(xd)
+        torch.cuda.synchronize()
+        dev = ok(cu.cuDeviceGet(torch.cuda.current_device()))
+        sms = ok(cu.cuDeviceGetDevResource(dev, cu.CUdevResourceType.CU_DEV_RESOURCE_TYPE_SM))
+        groups = ok(cu.cuDevSmResourceSplitByCount(1, sms, 0, 64))[0]
+        desc = ok(cu.cuDevResourceGenerateDesc([groups[0]], 1))
+        ctx = ok(cu.cuGreenCtxCreate(desc, dev, cu.CUgreenCtxCreate_flags.CU_GREEN_CTX_DEFAULT_STREAM))
+        stream = ok(cu.cuGreenCtxStreamCreate(ctx, cu.CUstream_flags.CU_STREAM_NON_BLOCKING, 0))
+        try:
+            layer.forward_ptr(xd.data_ptr(), 3, out.data_ptr(), 0, int(stream))
+            ok((cu.cuStreamSynchronize(stream)[0], None))
+            layer.check_device_status()
+            assert layer.launch_count() > 1
+        finally:
+            cu.cuStreamDestroy(stream)
+            cu.cuGreenCtxDestroy(ctx)
+        assert_parity(from_dev(out, np.uint16), ref.out_f32, what=spec.name)
+        layer.forward_ptr(xd.data_ptr(), 3, out.data_ptr())      # the whole device again
+        torch.cuda.synchronize()
+        assert layer.launch_count() == 1
+        assert_parity(from_dev(out, np.uint16), ref.out_f32, what=spec.name)
+    finally:
+        layer.close()
