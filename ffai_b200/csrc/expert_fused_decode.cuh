@@ -29,7 +29,9 @@
 // routed experts, in fp32 for 8-bit ones and for the shared expert.  The MMA reads the latter as three bf16 terms whose sum is
 // the fp32 value (split3): three times the MMAs of down, no bit lost.
 //
-// The waits at the grid barriers are bounded; a CTA that gives up raises the error word and leaves.
+// The waits at the grid barriers are bounded; a CTA that gives up raises the error word and leaves.  The barrier word then holds a
+// partial count, so it also marks the barrier broken: later launches leave before they write an output, until the host, which
+// reads the error word, has reset both.
 #pragma once
 #include <type_traits>
 
@@ -48,7 +50,7 @@ constexpr int SHARED_U = MAX_ROWS;  // table slot of the shared expert
 constexpr int RED_PITCH = 20;       // floats per activation column of a 16-row partial: lanes (g, t) hit distinct banks
 constexpr int RED_BYTES = 56 * 1024;           // partial sums; also router and routing scratch
 constexpr int MAX_DOWN_ITEMS = 12;             // down items a CTA's range may touch
-constexpr uint32_t BARRIER_TRIES = 1u << 21;   // polls of about half a microsecond
+constexpr uint32_t BARRIER_POLLS = 1u << 21;   // of about half a microsecond each
 enum : uint32_t { ERR_GRID_BARRIER = 64 };
 
 // Where the weights of a cell lie.  STREAM: one run in MMA fragment order, words first (lane l's at l * 16), then the
@@ -101,6 +103,8 @@ struct Params {
     float* split;               // [2 * CTAs][16 * MAX_T] partial sums of down items that two or more CTAs share
     uint32_t* tickets;          // [H/16] zero before the first launch, zero again after each
     uint32_t* barrier;          // one word, zero before the first launch
+    uint32_t* broken;           // non-zero after a wait that was given up
+    uint32_t polls;             // limit of a wait
     uint32_t* error_word;
 };
 
@@ -397,6 +401,7 @@ FFAI_DEVINL void cell_dot(const Raw<BITS, G32, SRC>& r, uint32_t mask, uint32_t 
 // CTA 0 adds what is missing to 2^31, so the top bit of the word flips when all have arrived, whatever came before.
 struct GridBarrier {
     uint32_t* word;
+    uint32_t polls;
     uint32_t old;
     FFAI_DEVINL void arrive() {   // all threads of the CTA
         __syncthreads();
@@ -406,9 +411,9 @@ struct GridBarrier {
         }
     }
     FFAI_DEVINL bool wait(int* failed) {
-        if (threadIdx.x == 0) {
+        if (threadIdx.x == 0 && !*failed) {
             bool ok = false;
-            for (uint32_t i = 0; i < BARRIER_TRIES && !ok; ++i) {
+            for (uint32_t i = 0; i < polls && !ok; ++i) {
                 uint32_t now;
                 asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(word) : "memory");
                 ok = ((now ^ old) & 0x80000000u) != 0;
@@ -420,6 +425,11 @@ struct GridBarrier {
         return *failed == 0;
     }
 };
+
+FFAI_DEVINL void give_up(const Params& p) {
+    atomicExch(p.broken, 1u);
+    atomicExch(p.error_word, (uint32_t)ERR_GRID_BARRIER);
+}
 
 // Where one expert set's gate/up products come from and go to.
 struct GateUp {
@@ -594,13 +604,13 @@ fused_decode_kernel(const Params p) {
     float* red = reinterpret_cast<float*>(smem + L::red());
     const uint32_t x_u = dstr::smem_u32(smem + L::x());
     const int x_pitch = L::x_pitch(H);
-    GridBarrier bar{p.barrier, 0};
+    GridBarrier bar{p.barrier, p.polls, 0};
     uint32_t mask, expo;
     asm volatile("mov.u32 %0, 0x000F000F;" : "=r"(mask));
     asm volatile("mov.u32 %0, 0x43004300;" : "=r"(expo));
 
     // ── phase 1: router logits of experts blockIdx.x, + gridDim.x, ... ──
-    if (threadIdx.x == 0) tb->failed = 0;
+    const uint32_t broken = threadIdx.x == 0 ? __ldcg(p.broken) : 0;
     for (int i = threadIdx.x; i < (MAX_ROWS + 1) * MAX_T; i += THREADS) { tb->colw[i / MAX_T][i % MAX_T] = 0.0f; tb->pos[i / MAX_T][i % MAX_T] = -1; }
     const int my_experts = (int)blockIdx.x < E ? (E - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
     const int wb = p.rp.kind == 1 ? 4 : 2, lsh = p.rp.kind == 1 ? 4 : 3, line16 = 1 << lsh;   // bytes per router weight; 16-byte pieces per 64 of them
@@ -722,6 +732,7 @@ fused_decode_kernel(const Params p) {
         acc = warp_sum(acc);
         if (lane == 0) p.sh_gate_logit[warp] = acc;
     }
+    if (threadIdx.x == 0) tb->failed = broken != 0;   // the first wait looks at it
     bar.arrive();
     if (SBITS != 0) {
         // the shared expert takes every token
@@ -735,7 +746,7 @@ fused_decode_kernel(const Params p) {
         gate_up_phase<SB, false, ROWS, SH_TERMS>(a, T, H, tb, x_u, x_pitch, red, warp, lane, mask, expo);
     }
     if (!bar.wait(&tb->failed)) {
-        if (threadIdx.x == 0) atomicExch(p.error_word, (uint32_t)ERR_GRID_BARRIER);
+        if (threadIdx.x == 0) give_up(p);
         return;
     }
 
@@ -841,7 +852,7 @@ fused_decode_kernel(const Params p) {
     }
     bar.arrive();
     if (!bar.wait(&tb->failed)) {
-        if (threadIdx.x == 0) atomicExch(p.error_word, (uint32_t)ERR_GRID_BARRIER);
+        if (threadIdx.x == 0) give_up(p);
         return;
     }
     const int first_item = F0 / n_flat, n_items = flat > 0 ? (F1 - 1) / n_flat - first_item + 1 : 0;

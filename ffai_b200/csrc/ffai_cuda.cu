@@ -86,7 +86,8 @@ struct ffai_moe_layer {
     uint16_t* fd_inner = nullptr;            // [terms][fdec::MAX_ROWS, I] activation results
     uint16_t* fd_sh_inner = nullptr;         // [terms][fdec::MAX_T, Is]
     float* fd_split = nullptr;               // [2 * SMs][16 * fdec::MAX_T]
-    uint32_t* fd_sync = nullptr;             // grid barrier word, then one ticket per 16-row block of the output (self-resetting)
+    uint32_t* fd_sync = nullptr;             // grid barrier word, its "broken" mark, then one ticket per 16-row block of the output (self-resetting)
+    uint32_t fd_polls = fdec::BARRIER_POLLS; // limit of a grid barrier wait (option "decode_wait_polls")
     int opt_decode = 0;              // decode kernels: 0 automatic, 1 per-lane cp.async rings, 2 bulk-copy streams
     int opt_overlap = 1;             // shared expert on a second stream beside router / plan / exchange (0: one stream)
     cudaStream_t aux_stream = nullptr;
@@ -898,11 +899,11 @@ extern "C" FFAI_API int ffai_moe_create(const ffai_moe_config* config, ffai_moe_
     if (L->fused_planned) {   // without room for its buffers the layer keeps to the launch chain
         const int terms = c.expert_bits == 8 ? fdec::INNER_TERMS<8> : fdec::INNER_TERMS<4>;
         if (ws_alloc(L, &L->fd_inner, terms * fdec::MAX_ROWS * I) || ws_alloc(L, &L->fd_sh_inner, (size_t)fdec::SH_TERMS * fdec::MAX_T * c.shared_intermediate) ||
-            ws_alloc(L, &L->fd_split, (size_t)2 * L->n_sms * 16 * fdec::MAX_T) || ws_alloc(L, &L->fd_sync, 1 + H / 16)) {
+            ws_alloc(L, &L->fd_split, (size_t)2 * L->n_sms * 16 * fdec::MAX_T) || ws_alloc(L, &L->fd_sync, 2 + H / 16)) {
             L->fused_planned = false;
             cudaGetLastError();
         } else {
-            CUDA_TRY(L, cudaMemset(L->fd_sync, 0, (1 + H / 16) * 4));
+            CUDA_TRY(L, cudaMemset(L->fd_sync, 0, (2 + H / 16) * 4));
         }
     }
     return FFAI_OK;
@@ -1234,6 +1235,11 @@ extern "C" FFAI_API int ffai_moe_set_option(ffai_moe_layer* L, const char* name,
         L->ep_wait_ns = (uint64_t)value * 1000000ull;
         return FFAI_OK;
     }
+    if (!strcmp(name, "decode_wait_polls")) {
+        if (value < 0) return fail(L, FFAI_ERR_INVALID_ARG, "option decode_wait_polls must be >= 0");
+        L->fd_polls = value;
+        return FFAI_OK;
+    }
     if (!strcmp(name, "decode")) {
         if (value < 0 || value > 2) return fail(L, FFAI_ERR_INVALID_ARG, "option decode must be 0 (automatic), 1 (cp.async rings) or 2 (bulk-copy streams)");
         L->opt_decode = value;
@@ -1287,7 +1293,7 @@ extern "C" FFAI_API int ffai_moe_check_device_status(ffai_moe_layer* L) {
     CUDA_TRY(L, cudaMemcpy(&word, L->error_word, 4, cudaMemcpyDeviceToHost));
     if (word) {
         CUDA_TRY(L, cudaMemset(L->error_word, 0, 4));
-        if (L->fd_sync) CUDA_TRY(L, cudaMemset(L->fd_sync, 0, (1 + L->cfg.hidden / 16) * 4));   // a barrier that was given up left a partial count
+        if (L->fd_sync) CUDA_TRY(L, cudaMemset(L->fd_sync, 0, (2 + L->cfg.hidden / 16) * 4));   // a barrier that was given up left a partial count
         return fail(L, FFAI_ERR_DEVICE_CHECK, "a kernel gave up a bounded wait (code %u)", word);
     }
     return FFAI_OK;
@@ -1707,7 +1713,7 @@ int forward_device(ffai_moe_layer* L, const uint16_t* x, int T, uint16_t* out, c
         p.inner = L->fd_inner; p.sh_inner = L->fd_sh_inner;
         p.inner_plane = fdec::MAX_ROWS * (uint32_t)I; p.sh_plane = fdec::MAX_T * (uint32_t)c.shared_intermediate;
         p.residual = residual; p.out = out;
-        p.split = L->fd_split; p.barrier = L->fd_sync; p.tickets = L->fd_sync + 1; p.error_word = L->error_word;
+        p.split = L->fd_split; p.barrier = L->fd_sync; p.broken = L->fd_sync + 1; p.tickets = L->fd_sync + 2; p.polls = L->fd_polls; p.error_word = L->error_word;
         cudaError_t status;
         const CoopLaunch done = launch_fused_decode(p, c.expert_bits, c.expert_group_size == 32, c.shared_intermediate > 0 ? c.shared_bits : 0, L->n_sms, st, &status);
         if (done == CoopLaunch::failed) return fail(L, FFAI_ERR_CUDA, "one-launch decode failed to launch: %s", cudaGetErrorString(status));
@@ -2208,7 +2214,8 @@ extern "C" FFAI_API int ffai_moe_forward_host(ffai_moe_layer* L, const uint16_t*
     if (n_chunks > 1) CUDA_TRY(L, cudaStreamSynchronize(L->d2h_stream));
     if (*pin_err) {
         cudaMemsetAsync(L->error_word, 0, 4, st);
-        if (L->fd_sync) cudaMemsetAsync(L->fd_sync, 0, (1 + L->cfg.hidden / 16) * 4, st);
+        if (L->fd_sync) cudaMemsetAsync(L->fd_sync, 0, (2 + L->cfg.hidden / 16) * 4, st);
+        cudaStreamSynchronize(st);   // the next call may be on another stream
         return fail(L, FFAI_ERR_DEVICE_CHECK, "a kernel gave up a bounded wait (code %u)", *pin_err);
     }
     if (!out_pinned && bytes) memcpy(out, L->pin_out, bytes);

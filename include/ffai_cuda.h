@@ -311,6 +311,9 @@ FFAI_API uint32_t ffai_ep_plan_exchange(const uint32_t* recv_counts, int32_t wor
  *   "overlap"      shared expert on a second stream beside router, plan and row exchange (default 1; 0: one stream)
  *   "pdl"          decode chain launched as programmatic dependent launches (default 1; 0: plain launches)
  *   "ep_wait_ms"   limit of a barrier wait of the peer-memory exchange, milliseconds (default 2000)
+ *   "decode_wait_polls"  one-launch decode: polls of a grid barrier, half a microsecond each, before a wait is given up
+ *                  (default 2097152).  Calls after that produce no output until the status was checked (see
+ *                  ffai_moe_check_device_status)
  *   "timeline"     1: the gate/up tcgen05 kernel records its device timeline (builds with FFAI_G100_TIMELINE only) */
 FFAI_API int ffai_moe_set_option(ffai_moe_layer* layer, const char* name, int32_t value);
 

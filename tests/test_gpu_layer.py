@@ -671,3 +671,47 @@ def test_stream_with_a_part_of_the_sms_takes_the_launch_chain(oracle_mod):
         assert_parity(from_dev(out, np.uint16), ref.out_f32, what=spec.name)
     finally:
         layer.close()
+
+
+@pytest.mark.parametrize("polls", [0, 1])
+def test_grid_barrier_that_is_given_up(oracle_mod, polls):
+    """The wait runs out (no poll, or one right after arriving): the call and the calls queued behind it write no output, the status
+    check reports it, and the next call is right again."""
+    import torch
+    spec = synth.LayerSpec("given_up", 1024, 512, 16, 4, expert_bits=8)
+    host = synth.make_layer(spec, 51)
+    x = synth.make_tokens(3, spec.hidden, 51)
+    ref = oracle_mod.moe_forward(host, x)
+    layer = MoELayer(host, 8)
+    try:
+        xd = to_dev(x)
+        out = torch.full_like(xd, 77)
+
+        def call():
+            layer.forward_ptr(xd.data_ptr(), 3, out.data_ptr())
+            assert layer.launch_count() == 1
+            torch.cuda.synchronize()
+        call()
+        assert_parity(from_dev(out, np.uint16), ref.out_f32, what=spec.name)
+        out.fill_(77)
+        layer.set_option("decode_wait_polls", polls)
+        call()
+        assert bool((out == 77).all())
+        layer.set_option("decode_wait_polls", 1 << 21)
+        call()
+        call()
+        assert bool((out == 77).all())
+        with pytest.raises(capi.FFAICudaError) as ei:
+            layer.check_device_status()
+        assert ei.value.status == capi.FFAI_ERR_DEVICE_CHECK
+        layer.check_device_status()
+        call()
+        assert_parity(from_dev(out, np.uint16), ref.out_f32, what=spec.name)
+        # the host entry checks by itself
+        layer.set_option("decode_wait_polls", polls)
+        with pytest.raises(capi.FFAICudaError):
+            layer.forward_host(x)
+        layer.set_option("decode_wait_polls", 1 << 21)
+        assert_parity(layer.forward_host(x)[0], ref.out_f32, what=spec.name)
+    finally:
+        layer.close()
