@@ -30,6 +30,8 @@ using namespace ffai;
 
 // ───────────────────────────── layer object ─────────────────────────────
 
+constexpr int NT2_COST = 12;   // default of option "nt2_cost"
+
 struct ffai_moe_layer {
     ffai_moe_config cfg{};
     int device = -1;
@@ -94,7 +96,7 @@ struct ffai_moe_layer {
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     int opt_pdl = 1;                 // decode chain: programmatic dependent launches (0: plain launches)
     int opt_decode_team = 0;         // bulk-copy streams: warps per 16-row block (0 automatic, 1, 4, 16)
-    int opt_nt2_cost = 12;           // bulk-copy streams: schedule weight of an item with more than 8 rows (8 = as one with fewer)
+    int opt_nt2_cost = NT2_COST;           // bulk-copy streams: schedule weight of an item with more than 8 rows (8 = as one with fewer)
     uint32_t* sb_gate = nullptr;     // repacked (scale | bias << 16) words of the expert projections
     uint32_t* sb_up = nullptr;
     uint32_t* sb_down = nullptr;
@@ -1679,9 +1681,11 @@ int forward_device(ffai_moe_layer* L, const uint16_t* x, int T, uint16_t* out, c
     }
 
     // The smallest batches: the whole block in one launch.  Stage events need launches to sit between, and the options
-    // that pick or tune one of the other decode kernels mean those kernels.
+    // that pick or tune other kernels mean those kernels.
+    const bool other_kernels = L->opt_path != 0 || L->opt_tc_min_rows != 0 || L->opt_decode != 0 || L->opt_ksplit != 0 || L->opt_decode_team != 0 ||
+                               L->opt_nt2_cost != NT2_COST;
     if (T <= fdec::MAX_T && M <= fdec::MAX_ROWS && L->fused_planned && (L->st_gate_up || c.expert_bits == 8 || c.expert_group_size == 32) &&
-        (L->opt_path == 0 || L->opt_path == 3) && L->opt_decode == 0 && L->opt_ksplit == 0 && L->opt_decode_team == 0 && !L->timing) {
+        !other_kernels && !L->timing) {
         fdec::Params p{};
         p.rp = router_params(L);
         p.x = x; p.xr = L->router_x ? L->router_x : x;

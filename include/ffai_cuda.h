@@ -293,8 +293,10 @@ FFAI_API uint32_t ffai_ep_plan_exchange(const uint32_t* recv_counts, int32_t wor
 
 /* Execution options, replacing the reference's FFAI_MOE_* environment switches
  * (Sources/FFAI/Models/MoELayer.swift:486-497).  Names:
- *   "path"         0 automatic, 1 CUDA-core grouped GEMV only, 2 tcgen05 grouped GEMM whenever possible,
- *                  3 streaming decode kernels whenever possible
+ *   "path"         0 automatic (up to 8 tokens and 64 routed rows of 4- and 8-bit experts: the whole block in one launch,
+ *                  unless stage timing is on or "tc_min_rows", "ksplit", "decode", "decode_team" or "nt2_cost" is
+ *                  set), 1 CUDA-core grouped GEMV only, 2 tcgen05 grouped GEMM whenever possible, 3 streaming
+ *                  decode kernels whenever possible
  *   "tc_min_rows"  smallest T*k that takes the tcgen05 path under "path" = 0 (0: default)
  *   "tc_weights"   tcgen05 path reads 0 automatic (the bf16 weight cache when the layer keeps one, except 4-bit experts
  *                  with few rows each: gate/up to 136, down to 112), 1 always the packed weights (4-bit only),
@@ -303,9 +305,7 @@ FFAI_API uint32_t ffai_ep_plan_exchange(const uint32_t* recv_counts, int32_t wor
  *                  overlap the compute (same bits: tokens are independent), 1 = always as one piece, 2..4 = at
  *                  most that many chunks
  *   "ksplit"       cp.async decode kernels: slices of the reduction axis per 16-row block (0 automatic, 1, 2, 4)
- *   "decode"       decode kernels: 0 automatic (up to 8 tokens and 64 routed rows, 4- and 8-bit experts: the whole block in
- *                  one launch, unless stage timing is on or "ksplit" / "decode_team" is set), 1 cp.async rings, 2 bulk-copy
- *                  streams
+ *   "decode"       decode kernels: 0 automatic, 1 cp.async rings, 2 bulk-copy streams
  *   "decode_team"  bulk-copy streams: warps that share one 16-row block (0 automatic, 1, 4, 16)
  *   "nt2_cost"     bulk-copy streams: schedule weight of a block with more than 8 rows, 8 = as one with fewer (8..32)
  *   "overlap"      shared expert on a second stream beside router, plan and row exchange (default 1; 0: one stream)

@@ -269,8 +269,8 @@ def test_tc_weight_cache_with_ragged_row_blocks(oracle_mod):
 def test_tc_cache_and_packed_weights_agree(oracle_mod):
     spec = synth.LayerSpec("cache_vs_packed", 512, 256, 16, 4, prefill_weight_cache=2)
     host = synth.make_layer(spec, 3)
-    x = synth.make_tokens(400, spec.hidden, 3)
-    layer = MoELayer(host, 400)
+    x = synth.make_tokens(500, spec.hidden, 3)          # 125 rows per expert: between the limits of down (112) and gate/up (136)
+    layer = MoELayer(host, 500)
     try:
         layer.set_option("path", TC)
         layer.set_option("tc_weights", 2)
@@ -380,7 +380,7 @@ def test_mma_group_size_32_gptoss_as_transcoded(oracle_mod, T):
     """GPT-OSS experts as the MXFP4 transcode leaves them: 4-bit, group 32, row biases; both pass widths."""
     spec = synth.cfg2_gptoss().with_(name="gptoss_gs32", expert_group_size=32, expert_row_bias=1)
     run_and_check(oracle_mod, spec, T, path=MMA)
-    run_and_check(oracle_mod, spec, T)                      # the automatic choice takes the same kernels
+    run_and_check(oracle_mod, spec, T)                      # the automatic choice: the same kernels from 9 tokens on
 
 
 def test_mma_group_size_32_small_shapes(oracle_mod):
@@ -402,16 +402,55 @@ def test_mma_every_reduction_split(oracle_mod, ksplit, gs):
 def test_auto_path_is_deterministic_and_matches_forced_paths(oracle_mod):
     spec = synth.cfg2_gptoss()
     host = synth.make_layer(spec, 0)
-    x = synth.make_tokens(8, spec.hidden, 0)
-    layer = MoELayer(host, 8)
+    x = synth.make_tokens(9, spec.hidden, 0)
+    layer = MoELayer(host, 9)
     try:
         a, _ = layer.forward_host(x)
         b, _ = layer.forward_host(x)
+        small, _ = layer.forward_host(x[:8])
+        again, _ = layer.forward_host(x[:8])
+        assert layer.launch_count() == 1
         layer.set_option("path", MMA)
         c, _ = layer.forward_host(x)
+        forced, _ = layer.forward_host(x[:8])
+        assert layer.launch_count() > 1
     finally:
         layer.close()
     assert np.array_equal(a, b) and np.array_equal(a, c)   # small batches take the streaming kernels
+    assert np.array_equal(small, again)
+    # the smallest ones the one-launch kernel: fp32 sums in another order, about 1e-5 of the RMS, which turn few bf16 roundings (of
+    # the activation's results, one in 1000, and of the outputs), each by at most 2**-7 of a value
+    fa, fb = synth.bf16_to_f32(small).astype(np.float64), synth.bf16_to_f32(forced).astype(np.float64)
+    assert 0 < np.sqrt(((fa - fb) ** 2).mean()) / np.sqrt((fb ** 2).mean()) < 1e-3
+
+
+@pytest.mark.parametrize("option", [("decode", 1), ("decode", 2), ("path", MMA), ("nt2_cost", 8), ("tc_min_rows", 64), ("decode_team", 4)])
+def test_options_of_other_kernels_keep_them_for_the_smallest_batches(oracle_mod, option):
+    spec = synth.LayerSpec("other_kernels", 512, 256, 16, 4)
+    host = synth.make_layer(spec, 61)
+    layer = MoELayer(host, 8)
+    try:
+        run_and_check(oracle_mod, spec, 8, layer=layer, host=host)
+        assert layer.launch_count() == 1
+        for T in (1, 3, 8):
+            run_and_check(oracle_mod, spec, T, layer=layer, host=host, options=dict([option]))
+            assert layer.launch_count() > 1
+    finally:
+        layer.close()
+
+
+@pytest.mark.parametrize("gs", [32, 64])
+@pytest.mark.parametrize("T", [6, 7])
+def test_one_launch_ends_where_the_token_rows_do_not_fit(oracle_mod, gs, T):
+    """Rows of 7168 take 16 KB of shared memory each: six fit beside the rest, the seventh does not."""
+    spec = synth.LayerSpec("long_rows", 7168, 64, 8, 2, expert_group_size=gs)
+    host = synth.make_layer(spec, 71)
+    layer = MoELayer(host, 8)
+    try:
+        run_and_check(oracle_mod, spec, T, layer=layer, host=host)
+        assert (layer.launch_count() == 1) == (T == 6)
+    finally:
+        layer.close()
 
 
 # ── Gemma-4-style routing: scaled logits, per-expert combine scale, GELU-GLU, the router's own input ──
