@@ -305,6 +305,24 @@ def run_prep(args):
                                    "algorithmic_bytes_per_launch": nbytes, "kernel_ms": ms}}), flush=True)
 
 
+def decode_roofline(spec, n_tokens, distinct, ms_step, stage_ms, peaks, traffic):
+    """Bytes and time of the dominant decode kernel: the gate/up product (2 of the 3 projections' bytes), or, where a step is one
+    launch (``stage_ms`` is None), that launch and all the bytes of the step.  ``traffic`` was measured on the gate/up kernel."""
+    H, bpw = spec.hidden, spec.bytes_per_weight()
+    one = stage_ms is None
+    kms = ms_step if one else stage_ms["gate_up"]
+    alg_bytes = spec.decode_bytes(n_tokens, distinct) if one else distinct * 2.0 * H * spec.intermediate * bpw + n_tokens * H * 2.0
+    achieved = alg_bytes / (kms * 1e-3) / 1e9
+    roofline = {"bound": "hbm", "kernel": "one_launch" if one else "gate_up", "achieved": achieved, "peak": peaks["hbm_gbs"],
+                "unit": "GB/s", "frac": achieved / peaks["hbm_gbs"], "peak_source": peaks["source"],
+                "traffic": None if one else traffic, "algorithmic_bytes_per_launch": alg_bytes, "kernel_ms": kms}
+    if not one:
+        down_bytes = distinct * H * spec.intermediate * bpw + n_tokens * spec.top_k * (spec.intermediate * 2.0 + H * 4.0)
+        roofline["down"] = {"kernel_ms": stage_ms["down"], "algorithmic_bytes_per_launch": down_bytes,
+                            "frac": down_bytes / (stage_ms["down"] * 1e-3) / 1e9 / peaks["hbm_gbs"]}
+    return roofline
+
+
 def measure(name, args, rank, local_rank, world, dist, steps, with_clocks):
     """Times one workload on this process's GPU (with `world` > 1 and a sharding rule: together with the
     other ranks).  Returns the result record on rank 0, None elsewhere."""
@@ -383,24 +401,27 @@ def measure(name, args, rank, local_rank, world, dist, steps, with_clocks):
     sampler = ClockSampler(local_rank) if (with_clocks and rank == 0) else None
     if sampler:
         sampler.start()
-    times, stages, launches = [], [], 0
+    times, stages, launches, one_launch = [], [], 0, True
     for i in range(steps):
         ms, _, nl = step(i, True)
         times.append(ms); launches += nl
+        one_launch = one_launch and nl == 1
         if ep_mode:
             sync_all()
     sync_all()
     clocks = sampler.stop() if sampler else None
 
     # per-kernel durations for the roofline: a second pass with the library's stage events switched on
-    # (the event records cost a few microseconds per stage, so they stay out of the headline pass)
-    layer.set_stage_timing(True)
-    for i in range(min(steps, 20)):
-        _, st, nl = step(i, True)
-        stages.append(st); launches += nl
-        if ep_mode:
-            sync_all()
-    layer.set_stage_timing(False)
+    # (the event records cost a few microseconds per stage, so they stay out of the headline pass).  A step that is one
+    # launch has no stages: with events on, the library runs other kernels.
+    if not one_launch:
+        layer.set_stage_timing(True)
+        for i in range(min(steps, 20)):
+            _, st, nl = step(i, True)
+            stages.append(st); launches += nl
+            if ep_mode:
+                sync_all()
+        layer.set_stage_timing(False)
 
     # end to end through the host-buffer entry point (copies inside the timed region)
     e2e_times = []
@@ -432,20 +453,10 @@ def measure(name, args, rank, local_rank, world, dist, steps, with_clocks):
         peaks = measured_peaks()
         used = [distinct[i % N_BATCHES] for i in range(steps)]
         mean_distinct = statistics.mean(used)
-        stage_mean = {k: statistics.mean(s[k] for s in stages) for k in stages[0]}
-        bpw = spec.bytes_per_weight()
+        stage_mean = {k: statistics.mean(s[k] for s in stages) for k in stages[0]} if stages else None
         step_tokens = n_tokens * world if (ep_mode or sharding is None) else n_tokens
         if regime == "decode":
-            # dominant kernel: the fused gate/up product (2 of the 3 projections' bytes)
-            kernel, kms = "gate_up", stage_mean["gate_up"]
-            alg_bytes = mean_distinct * 2.0 * spec.hidden * spec.intermediate * bpw + n_tokens * H * 2.0
-            achieved = alg_bytes / (kms * 1e-3) / 1e9
-            roofline = {"bound": "hbm", "kernel": kernel, "achieved": achieved, "peak": peaks["hbm_gbs"],
-                        "unit": "GB/s", "frac": achieved / peaks["hbm_gbs"], "peak_source": peaks["source"],
-                        "traffic": ncu_traffic(name), "algorithmic_bytes_per_launch": alg_bytes, "kernel_ms": kms}
-            down_bytes = mean_distinct * spec.hidden * spec.intermediate * bpw + n_tokens * spec.top_k * (spec.intermediate * 2.0 + H * 4.0)
-            roofline["down"] = {"kernel_ms": stage_mean["down"], "algorithmic_bytes_per_launch": down_bytes,
-                                "frac": down_bytes / (stage_mean["down"] * 1e-3) / 1e9 / peaks["hbm_gbs"]}
+            roofline = decode_roofline(spec, n_tokens, mean_distinct, ms_step, stage_mean, peaks, ncu_traffic(name))
             layer_bytes = spec.decode_bytes(n_tokens, mean_distinct)
             layer_frac = layer_bytes / (ms_step * 1e-3) / 1e9 / peaks["hbm_gbs"]
         else:

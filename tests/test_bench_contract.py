@@ -45,3 +45,15 @@ def test_reference_arm_under_a_multi_rank_launch_only_rank_zero_prints():
                          stdin=subprocess.DEVNULL)
     assert out.returncode == 0, out.stderr[-2000:]
     assert not [ln for ln in out.stdout.splitlines() if ln.startswith("{")]
+
+
+def test_decode_roofline_names_the_kernel_that_the_step_launches():
+    import bench
+    from ffai_b200 import synth
+    spec = synth.cfg2_gptoss()
+    peaks = {"hbm_gbs": 6500.0, "source": "given"}
+    one = bench.decode_roofline(spec, 1, 4.0, 0.03, None, peaks, {"dram": 1})
+    assert one["kernel"] == "one_launch" and one["kernel_ms"] == 0.03 and "down" not in one and one["traffic"] is None
+    assert one["algorithmic_bytes_per_launch"] == spec.decode_bytes(1, 4.0)
+    chain = bench.decode_roofline(spec, 64, 32.0, 0.15, {"gate_up": 0.08, "down": 0.04}, peaks, {"dram": 1})
+    assert chain["kernel"] == "gate_up" and chain["kernel_ms"] == 0.08 and chain["down"]["kernel_ms"] == 0.04 and chain["traffic"] == {"dram": 1}
