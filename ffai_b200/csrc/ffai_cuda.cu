@@ -22,6 +22,7 @@
 #include "expert_stream_decode.cuh"
 #include "plan.cuh"
 #include "router.cuh"
+#include "router_tiles.hpp"
 #include "safetensors.hpp"
 #include "tc_path.cuh"
 #include "weight_prep.cuh"
@@ -349,10 +350,7 @@ int launch_router_batched(const RouterParams& p, const uint16_t* x, int T, uint3
     // hidden axis into ranges of chunks as well and leave the ordered sum of the chunks to the routing kernel.
     if ((p.kind == FFAI_LINEAR_F32 || p.kind == FFAI_LINEAR_BF16) && p.hidden % 64 == 0 && T >= 256) {
         const int tiles = ((T + RB_TOK - 1) / RB_TOK) * ((p.n_experts + RB_EXP - 1) / RB_EXP);
-        // Twice as wide tiles, one block per SM, from the batch on that gives more than half of the SMs one (below that the
-        // narrow tiles, one per SM, take less); a last column of at most 64 experts would leave half a wide tile empty.
-        const int wide = tiles / 2;
-        if (((p.n_experts + RB_EXP - 1) / RB_EXP) % 2 == 0 && wide * 2 > n_sms) {
+        if (((p.n_experts + RB_EXP - 1) / RB_EXP) % 2 == 0 && router_wide_tiles(tiles, n_sms, p.kind == FFAI_LINEAR_F32)) {
             const dim3 grid((T + RB_TOK - 1) / RB_TOK, (p.n_experts + RW_EXP - 1) / RW_EXP);
             static SmemOptIn opt1, opt2;
             bool ok;

@@ -574,7 +574,7 @@ def test_one_launch_decode(oracle_mod, name, T, kw, residual):
 # ── the wide router projection (128 tokens x 128 experts per block): ragged last tiles both ways, one chunk and three ──
 
 @pytest.mark.parametrize("kind", [capi.LINEAR_F32, capi.LINEAR_BF16])
-@pytest.mark.parametrize("T,E,H", [(1201, 1000, 192), (4800, 193, 64)])
+@pytest.mark.parametrize("T,E,H", [(1201, 1000, 192), (4800, 193, 64), (2500, 1000, 64)])     # the last: an odd count of rounds, narrow tiles
 def test_wide_router_tiles(oracle_mod, kind, T, E, H):
     spec = synth.LayerSpec("wide_router_tiles", hidden=H, intermediate=64, n_experts=E, top_k=2, router_kind=kind, router_has_bias=1)
     mask = np.zeros(T, dtype=np.uint8)
