@@ -1294,6 +1294,7 @@ extern "C" FFAI_API int ffai_moe_check_device_status(ffai_moe_layer* L) {
     if (word) {
         CUDA_TRY(L, cudaMemset(L->error_word, 0, 4));
         if (L->fd_sync) CUDA_TRY(L, cudaMemset(L->fd_sync, 0, (2 + L->cfg.hidden / 16) * 4));   // a barrier that was given up left a partial count
+        CUDA_TRY(L, cudaDeviceSynchronize());   // the next call may be on a stream that does not wait for these
         return fail(L, FFAI_ERR_DEVICE_CHECK, "a kernel gave up a bounded wait (code %u)", word);
     }
     return FFAI_OK;

@@ -754,3 +754,29 @@ def test_grid_barrier_that_is_given_up(oracle_mod, polls):
         assert_parity(layer.forward_host(x)[0], ref.out_f32, what=spec.name)
     finally:
         layer.close()
+
+
+@pytest.mark.parametrize("bits,gs", [(4, 64), (4, 32), (8, 64)])
+def test_one_launch_in_a_captured_graph(oracle_mod, bits, gs):
+    import torch
+    spec = synth.LayerSpec("captured", 512, 256, 16, 4, expert_bits=bits, expert_group_size=gs)
+    host = synth.make_layer(spec, 91)
+    layer = MoELayer(host, 8)
+    try:
+        x = torch.zeros(5, spec.hidden, dtype=torch.int16, device="cuda")
+        out = torch.zeros_like(x)
+        graph = torch.cuda.CUDAGraph()
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph):       # the handle's first call
+            layer.forward_ptr(x.data_ptr(), 5, out.data_ptr(), 0, torch.cuda.current_stream().cuda_stream)
+        assert layer.launch_count() == 1
+        for seed in (1, 2, 3):
+            rows = synth.make_tokens(5, spec.hidden, seed)
+            x.copy_(to_dev(rows))
+            graph.replay()
+            torch.cuda.synchronize()
+            assert_parity(from_dev(out, np.uint16), oracle_mod.moe_forward(host, rows).out_f32, what=spec.name)
+        layer.check_device_status()
+        del graph
+    finally:
+        layer.close()
