@@ -116,7 +116,8 @@ FFAI_DEVINL void warp_argbest(float& v, int& i) {
 }
 
 // Top-k of vals[0..E) in shared memory by one warp; selected indices (in
-// selection order) returned lane-wise: lane j < k holds index j.
+// selection order) returned lane-wise: lane j < k holds index j.  A NaN counts as -inf: an expert
+// whose logit is undefined is selected only when no other is left, as where values are compared with `>`.
 //
 // Up to 32 * NV values: every lane keeps its strided values (e = lane + 32 j) as order-preserving integer keys in
 // registers and a round is two warp reductions in hardware (largest key, then smallest index among its holders);
@@ -129,8 +130,8 @@ FFAI_DEVINL void warp_topk_regs(const float* vals, int E, int k, int lane, int& 
         const int e = lane + 32 * j;
         key[j] = 0u;
         if (e < E) {
-            const uint32_t b = __float_as_uint(vals[e] + 0.0f);   // -0 and +0 are one value
-            key[j] = max((b & 0x80000000u) ? ~b : (b | 0x80000000u), 1u);
+            const uint32_t b = __float_as_uint(fmaxf(vals[e], -INFINITY) + 0.0f);   // NaN is -inf; -0 and +0 are one value
+            key[j] = (b & 0x80000000u) ? ~b : (b | 0x80000000u);                    // at least 0x007FFFFF
         }
     }
     uint32_t best = 0u, at = 0x7FFFFFFFu;
@@ -171,13 +172,14 @@ FFAI_DEVINL void warp_topk(const float* vals, int E, int k, int lane, int& my_id
         int bi = -1;
         for (int j = 0, e = lane; e < E; ++j, e += 32) {
             if (taken & (1u << j)) continue;
-            float v = vals[e];
+            const float v = fmaxf(vals[e], -INFINITY);
             if (bi < 0 || v > bv) { bv = v; bi = e; }
         }
         warp_argbest(bv, bi);
         if (bi >= 0 && (bi & 31) == lane) taken |= 1u << (bi >> 5);
-        if (lane == r) { my_idx = bi; my_val = bv; }
+        if (lane == r) my_idx = bi;
     }
+    if (lane < k) my_val = vals[my_idx];
 }
 
 // Routing of one token by one warp, given its logits in shared memory.

@@ -756,6 +756,27 @@ def test_grid_barrier_that_is_given_up(oracle_mod, polls):
         layer.close()
 
 
+@pytest.mark.parametrize("E", [32, 100, 256, 300])
+@pytest.mark.parametrize("gating", [capi.GATING_SOFTMAX_THEN_TOPK, capi.GATING_TOPK_THEN_SOFTMAX])
+def test_an_undefined_logit_is_not_selected(oracle_mod, E, gating):
+    """One expert's router row is NaN: every router kernel selects among the others, as comparing with `>` does (the expert is not
+    the first one, which the oracle's scan starts from)."""
+    spec = synth.LayerSpec("nan_logit", 256, 64, E, 4, gating_mode=gating, router_logits_bf16=0)
+    host = synth.make_layer(spec, 81)
+    host.arrays["gate.weight"][7] = 0x7FC0
+    layer = MoELayer(host, 300)
+    try:
+        for T in (1, 8, 40, 300):
+            x = synth.make_tokens(T, spec.hidden, T)
+            out, dbg = layer.forward_host(x, debug=True)
+            ref = oracle_mod.moe_forward(host, x)
+            assert not (ref.indices == 7).any()
+            assert np.array_equal(dbg.indices, ref.indices) and np.array_equal(dbg.weights, ref.weights)
+            assert_parity(out, ref.out_f32, what=spec.name)
+    finally:
+        layer.close()
+
+
 @pytest.mark.parametrize("bits,gs", [(4, 64), (4, 32), (8, 64)])
 def test_one_launch_in_a_captured_graph(oracle_mod, bits, gs):
     import torch
